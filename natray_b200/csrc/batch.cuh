@@ -397,7 +397,7 @@ static uint64_t enqueue_step_multi(Batch& B, uint32_t n_jobs, const uint32_t* to
     LM(k_solve_reset_m, GK_ONE, 32, s);
     // Every scene needs a CTA of the joint solve.
     const uint32_t solve_ctas = B.tune.solve_ctas ? std::min(B.ctas, std::max(B.tune.solve_ctas, n_jobs)) : B.ctas;
-    nl += enqueue_solve(S0, s, B.d_jobs, n_jobs, fp64, prof, solve_ctas);
+    nl += enqueue_solve(S0, s, B.d_jobs, n_jobs, fp64, prof, solve_ctas, SOLVE_DYN);
     LM(k_project_m, GK_CELL, 256, s);
     LM(k_extend_1_m, GK_CELL, 256, s);
     LM(k_extend_2_m, GK_CELL, 256, s);

@@ -127,7 +127,7 @@ struct Dev {
     int32_t* acc;
     float* cf;
     float* air[2];
-    double* xsum;   // the solver's running sums: 2 parities x 256 residues x 3 quantities
+    double* xsum;   // the solver's running sums: 2 parities x 3 quantities x 256 residues
     double* spart;  // the solver's per-block partial sums when a CTA has many blocks: 3 x cap_blocks
     float4* mem_x[2];
     float4* mem_v[2];
@@ -154,7 +154,7 @@ struct Dev {
     int32_t* tiles;     // per block: the P2G tile, 8 fields x 343 i32
     uint32_t* tile_ok;  // per block: 1 when its tile holds this step's sums
     uint32_t* coltot;   // radix sort: per digit, the elements with that digit
-    uint32_t* wnb;      // solver: per cell, its 6 neighbours that are water (or NONE), 8 words
+    uint32_t* wnb;      // solver: a record per block (2 KB) where a CTA's blocks do not fit its shared memory
 };
 
 // Where a CTA is in its scene's grid: x() and nx() as blockIdx.x and gridDim.x of a launch for

@@ -204,15 +204,15 @@ static ntr_status device_facts(int device, DevFacts& out) {
             // The persistent solver's grid must be co-resident: at most what occupancy allows,
             // for the one-scene and the many-scene solve alike. CTA c owns the blocks c (mod 256)
             // (and c + G, ... with fewer CTAs): at most 256.
+            // With the shared memory of the launches that keep block records there.
             int occ = 1 << 30, o = 0;
-            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_solve<true>, SOLVE_T, 0));
-            occ = std::min(occ, o);
-            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_solve<false>, SOLVE_T, 0));
-            occ = std::min(occ, o);
-            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_solve_batch<true>, SOLVE_T, 0));
-            occ = std::min(occ, o);
-            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_solve_batch<false>, SOLVE_T, 0));
-            occ = std::min(occ, o);
+            const void* solves[4] = {(const void*)k_solve<true>, (const void*)k_solve<false>, (const void*)k_solve_batch<true>,
+                                     (const void*)k_solve_batch<false>};
+            for (const void* k : solves) {
+                CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_DYN));
+                CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, SOLVE_T, SOLVE_DYN));
+                occ = std::min(occ, o);
+            }
             f.coop_ctas = (uint32_t)std::min(256, f.sms * occ);
             f.coop_all = (uint32_t)(f.sms * occ);
             CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_p2g, P2G_T, 0));
@@ -494,12 +494,13 @@ static ntr_status prof_report(Prof& prof, char* report, size_t cap, size_t* len)
 
 // The pressure solve as one cooperative launch of `ctas` CTAs on `s`: of S alone (jobs == NULL),
 // or of the `n_jobs` simulations whose pointer tables are at `jobs` on the device. Each job's
-// barrier counter must be zero (the step resets it before the launch).
-static uint64_t enqueue_solve(Sim& S, cudaStream_t s, const Dev* jobs, uint32_t n_jobs, bool fp64, Prof* prof, uint32_t ctas) {
+// barrier counter must be zero (the step resets it before the launch). `dyn`: shared memory for
+// the records of CTAs with more blocks than warps.
+static uint64_t enqueue_solve(Sim& S, cudaStream_t s, const Dev* jobs, uint32_t n_jobs, bool fp64, Prof* prof, uint32_t ctas, uint32_t dyn) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(SOLVE_T);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = dyn;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -525,13 +526,14 @@ struct Grids {
     uint32_t cell, p2g, g2p, solve;
     bool g2p_wide;  // G2P in CTAs of 256 threads (scenes under 300k particles), else 128
     uint32_t blk;   // CTAs of a scene's per-block kernels in a many-scene launch (a fixed stride)
+    uint32_t solve_dyn;  // the solve's shared memory for block records: none while every warp has at most one block
 };
 static Grids launch_grids(const Sim& S) {
     const bool wide = S.D.Np < 300000u;
     const uint32_t per_sm = S.tune.block_ctas_per_sm;
     Grids g{(uint32_t)S.sms * S.tune.cell_ctas_per_sm, (uint32_t)S.sms * std::min(per_sm, S.p2g_occ),
             (uint32_t)S.sms * std::min(per_sm, wide ? S.g2p256_occ : S.g2p128_occ),
-            S.tune.solve_ctas ? S.tune.solve_ctas : S.coop_ctas, wide, (uint32_t)S.sms * per_sm};
+            S.tune.solve_ctas ? S.tune.solve_ctas : S.coop_ctas, wide, (uint32_t)S.sms * per_sm, SOLVE_DYN};
     const uint32_t nb = S.size_class;
     if (nb) {
         g.cell = std::max(1u, std::min(g.cell, (nb * 64u + 255u) / 256u));
@@ -539,6 +541,8 @@ static Grids launch_grids(const Sim& S) {
         g.p2g = std::max(1u, std::min(g.p2g, nb));
         g.g2p = std::max(1u, std::min(g.g2p, nb));
         if (!S.tune.solve_ctas) g.solve = std::max(1u, std::min(g.solve, (nb + SOLVE_T / 32 - 1) / (SOLVE_T / 32)));
+        // (A scene that outgrows its class within a batch of steps keeps its records in D.wnb.)
+        if ((nb + 255u) / 256u * ((256u + g.solve - 1u) / g.solve) <= (uint32_t)SOLVE_W) g.solve_dyn = 0u;
     }
     return g;
 }
@@ -640,7 +644,7 @@ static uint64_t enqueue_step(Sim& S, cudaStream_t s, uint32_t n_mem, uint32_t n_
     L(k_bullet_finish, n_shots, 256, D);
     L(k_bullet_apply, G_cell, 256, D);
     // (k_bullet_apply has set the pressure solve's grid barrier counter to zero.)
-    n += enqueue_solve(S, s, nullptr, 1u, fp64, prof, grids.solve);
+    n += enqueue_solve(S, s, nullptr, 1u, fp64, prof, grids.solve, grids.solve_dyn);
     L(k_project, G_cell, 256, D);
     L(k_extend_1, G_cell, 256, D);
     L(k_extend_2, G_cell, 256, D);
