@@ -180,36 +180,64 @@ struct Near {
     float ax, ay, nx, ny, depth;
 };
 
-// The nearest point of bullet `bi`'s outline to q = (z, r) of its body frame
-// (bullet.wgsl:438-472). `ol` is the bullet's outline (in shared memory).
-__device__ Near nearest_surface(const float2* __restrict__ ol, float qx, float qy) {
-    float2 first = ol[0], last = ol[NTR_OUTLINE - 1];
+// A bullet's outline as the contact samples walk it, made once per CTA in shared memory: its points,
+// and the 34 segments of the closed outline (from the axis to the first point, between points, from
+// the last point to the axis): start and direction, squared length and its reciprocal.
+constexpr uint32_t OUTLINE_SEGS = NTR_OUTLINE + 1;
+struct Outline {
+    float2 pt[NTR_OUTLINE];
+    float4 seg[OUTLINE_SEGS];
+    float2 len[OUTLINE_SEGS];
+};
+__device__ __forceinline__ void outline_segment(Outline& o, const float2* __restrict__ ol, uint32_t j) {
+    const float2 first = ol[0], last = ol[NTR_OUTLINE - 1];
+    const float2 p0 = j > 0 ? ol[j - 1] : make_float2(first.x, 0.0f), p1 = j < NTR_OUTLINE ? ol[j] : make_float2(last.x, 0.0f);
+    const float ex = p1.x - p0.x, ey = p1.y - p0.y;
+    const float len2 = ex * ex + ey * ey;
+    o.seg[j] = make_float4(p0.x, p0.y, ex, ey);
+    o.len[j] = make_float2(len2, 1.0f / len2);
+    if (j < NTR_OUTLINE) o.pt[j] = ol[j];
+}
+
+// The nearest point of a bullet's outline to q = (z, r) of its body frame (bullet.wgsl:438-472).
+// The walk keeps only the first nearest segment, and what is wanted of it is worked out after: so
+// the segments' chains (a division and a square root each) do not depend on one another and run
+// four at a time. One by one, with the normal worked out at each new nearest, a walk took 14k
+// cycles, which was most of the contact search. The foot of the perpendicular is at
+// clamp(dot / len2, 0, 1) of the segment; the quotient by the kept reciprocal (div_by).
+__device__ __forceinline__ float2 outline_foot(float4 s, float2 len, float qx, float qy) {
+    const float tt = clampf_(div_by((qx - s.x) * s.z + (qy - s.y) * s.w, len.x, len.y), 0.0f, 1.0f);
+    return make_float2(s.x + s.z * tt, s.y + s.w * tt);
+}
+__device__ __forceinline__ Near nearest_surface(const Outline& ol, float qx, float qy) {
+    const float2 first = ol.pt[0], last = ol.pt[NTR_OUTLINE - 1];
     Near o = {qx, qy, 0.0f, 0.0f, 0.0f};
     float best = BIG_F;
-    for (uint32_t j = 0; j <= NTR_OUTLINE; j++) {
-        float2 p0 = make_float2(first.x, 0.0f), p1 = make_float2(last.x, 0.0f);
-        if (j > 0) p0 = ol[j - 1];
-        if (j < NTR_OUTLINE) p1 = ol[j];
-        float ex = p1.x - p0.x, ey = p1.y - p0.y;
-        float len2 = ex * ex + ey * ey;
-        if (len2 <= 0.0f) continue;
-        float tt = clampf_(((qx - p0.x) * ex + (qy - p0.y) * ey) / len2, 0.0f, 1.0f);
-        float onx = p0.x + ex * tt, ony = p0.y + ey * tt;
-        float dqx = qx - onx, dqy = qy - ony;
-        float d = sqrtf(dqx * dqx + dqy * dqy);
-        if (d < best) {
-            best = d;
-            o.ax = onx, o.ay = ony;
-            float nnx = -ey, nny = ex;
-            float inv = 1.0f / sqrtf(nnx * nnx + nny * nny);
-            o.nx = nnx * inv, o.ny = nny * inv;
-        }
+    uint32_t jb = NONE;
+    static_assert(OUTLINE_SEGS % 2 == 0, "the walk's unrolling");
+#pragma unroll 4
+    for (uint32_t j = 0; j < OUTLINE_SEGS; j++) {
+        const float2 len = ol.len[j], on = outline_foot(ol.seg[j], len, qx, qy);
+        const float dqx = qx - on.x, dqy = qy - on.y;
+        const float d = sqrtf(dqx * dqx + dqy * dqy);
+        if (len.x > 0.0f && d < best) best = d, jb = j;
+    }
+    if (jb != NONE) {
+        const float4 s = ol.seg[jb];
+        const float2 on = outline_foot(s, ol.len[jb], qx, qy);
+        o.ax = on.x, o.ay = on.y;
+        const float nnx = -s.w, nny = s.z;
+        const float inv = 1.0f / sqrtf(nnx * nnx + nny * nny);
+        o.nx = nnx * inv, o.ny = nny * inv;
     }
     bool inside = false;
     if (qx > first.x && qx < last.x) {
-        uint32_t k = 1;
-        while (k < NTR_OUTLINE - 1 && ol[k].x < qx) k++;
-        float2 a = ol[k - 1], c = ol[k];
+        // The first point from the second on that is not before qx, or the last.
+        uint32_t k = NTR_OUTLINE - 1;
+#pragma unroll 8
+        for (uint32_t m = NTR_OUTLINE - 2; m >= 1; m--)
+            if (!(ol.pt[m].x < qx)) k = m;
+        const float2 a = ol.pt[k - 1], c = ol.pt[k];
         float f = (qx - a.x) / mx(c.x - a.x, 1e-12f);
         inside = qy < a.y * (1.0f - f) + c.y * f;
     }
@@ -320,11 +348,11 @@ struct ContactHit {
     float share, depth;
 };
 
-// One sample against a bullet, `ol` its outline (the contact search of bullet.wgsl:426-611):
-// false if it does not count (no weight on this vertex, or beyond the bullet's reach). With
-// `hit`, also what the response needs.
-__device__ __forceinline__ bool contact_sample(const float2* ol, const ContactTri& t, uint32_t a, uint32_t c, const DBullet& b, V3 xb,
-                                               float4 back, V3 w, float band, float& depth, ContactHit* hit) {
+// One sample against a bullet, `ol` its outline (the contact search of bullet.wgsl:426-611), and
+// what the response needs of it: false if it does not count (no weight on this vertex, or beyond
+// the bullet's reach).
+__device__ __forceinline__ bool contact_sample(const Outline& ol, const ContactTri& t, uint32_t a, uint32_t c, const DBullet& b, V3 xb,
+                                               float4 back, V3 w, float band, ContactHit& hit) {
     const uint32_t n = t.n;
     V3 bary = v3((float)a, (float)c, (float)(n - a - c)) / (float)n;
     float wi = bary[t.own];
@@ -335,17 +363,14 @@ __device__ __forceinline__ bool contact_sample(const float2* ol, const ContactTr
     V3 q = qrot(back, r);
     float rho = sqrtf(q.x * q.x + q.y * q.y);
     Near nr = nearest_surface(ol, q.z, rho);
-    depth = nr.depth;
-    if (hit) {
-        float rx = 1.0f, ry = 0.0f;
-        if (rho > 1e-9f) rx = q.x / rho, ry = q.y / rho;
-        hit->depth = nr.depth;
-        hit->on_b = qrot(b.q, v3(rx * nr.ay, ry * nr.ay, nr.ax));
-        hit->gap = hit->on_b - r;
-        hit->nrm = qrot(b.q, v3(rx * nr.ny, ry * nr.ny, nr.nx));
-        hit->share = wi / dot(bary, bary);
-        hit->rel = bary.x * t.pv[0] + bary.y * t.pv[1] + bary.z * t.pv[2] - xyz(b.v) - cross(w, hit->on_b);
-    }
+    float rx = 1.0f, ry = 0.0f;
+    if (rho > 1e-9f) rx = q.x / rho, ry = q.y / rho;
+    hit.depth = nr.depth;
+    hit.on_b = qrot(b.q, v3(rx * nr.ay, ry * nr.ay, nr.ax));
+    hit.gap = hit.on_b - r;
+    hit.nrm = qrot(b.q, v3(rx * nr.ny, ry * nr.ny, nr.nx));
+    hit.share = wi / dot(bary, bary);
+    hit.rel = bary.x * t.pv[0] + bary.y * t.pv[1] + bary.z * t.pv[2] - xyz(b.v) - cross(w, hit.on_b);
     return true;
 }
 
@@ -354,10 +379,10 @@ __device__ __forceinline__ bool contact_sample(const float2* ol, const ContactTr
 // lane keeping the first of its samples of greatest depth, then the warp's: the greatest depth,
 // the earliest in the reference's order among equals. For finite depths that is the sample the
 // reference's sequential search ends on (it takes a sample only when deeper than the best so
-// far, from -band): found when its depth is above -band. Returns the sample's triangle slot and
-// index. All 32 lanes call it.
+// far, from -band): found when its depth is above -band. `hit`: the sample, from the lane that
+// worked it out. All 32 lanes call it.
 __device__ bool contact_search_warp(const Dev& D, int par, int src, uint32_t i_l, V3 x_l, V3 v_l, float band_l, float sub, const DBullet& b,
-                                    V3 xb, float4 back, V3 w, const float2* ol, uint32_t& k_best, uint32_t& m_best) {
+                                    V3 xb, float4 back, V3 w, const Outline& ol, ContactHit& hit) {
     const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
     const uint32_t i = __shfl_sync(full, i_l, src);
     const V3 x = {__shfl_sync(full, x_l.x, src), __shfl_sync(full, x_l.y, src), __shfl_sync(full, x_l.z, src)};
@@ -365,6 +390,7 @@ __device__ bool contact_search_warp(const Dev& D, int par, int src, uint32_t i_l
     const float band = __shfl_sync(full, band_l, src);
     const uint32_t k0 = D.vtri_off[i], k1 = D.vtri_off[i + 1];
     bool have = false;
+    ContactHit mine_hit = {};
     float bd = 0.0f;
     uint32_t bo = 0u;  // (k - k0) * 64 + sample: the reference's order
     // The triangles (and the vertex alone, last), 32 at a time: lane j loads the j-th, so their
@@ -403,14 +429,17 @@ __device__ bool contact_search_warp(const Dev& D, int par, int src, uint32_t i_l
             if (p >= total) continue;
             uint32_t a, c;
             contact_sample_ac(m, t.n, a, c);
-            float depth;
-            if (contact_sample(ol, t, a, c, b, xb, back, w, band, depth, nullptr) && (!have || depth > bd)) {
+            ContactHit h;
+            if (contact_sample(ol, t, a, c, b, xb, back, w, band, h) && (!have || h.depth > bd)) {
                 have = true;
-                bd = depth;
+                mine_hit = h;
+                bd = h.depth;
                 bo = (kb + j - k0) * 64u + m;
             }
         }
     }
+    const bool had = have;
+    const uint32_t my_bo = bo;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const bool oh = __shfl_xor_sync(full, have, o);
@@ -419,15 +448,17 @@ __device__ bool contact_search_warp(const Dev& D, int par, int src, uint32_t i_l
         if (oh && (!have || od > bd || (od == bd && oo < bo))) have = true, bd = od, bo = oo;
     }
     if (!have || !(bd > -band)) return false;
-    k_best = k0 + bo / 64u;
-    m_best = bo % 64u;
+    const int from = __ffs(__ballot_sync(full, had && my_bo == bo)) - 1;
+    auto take = [&](V3 v) { return V3{__shfl_sync(full, v.x, from), __shfl_sync(full, v.y, from), __shfl_sync(full, v.z, from)}; };
+    hit.on_b = take(mine_hit.on_b), hit.gap = take(mine_hit.gap), hit.nrm = take(mine_hit.nrm), hit.rel = take(mine_hit.rel);
+    hit.share = __shfl_sync(full, mine_hit.share, from), hit.depth = bd;
     return true;
 }
 
 // Contact of the rubber with the bullets (bullet.wgsl:426-611), for the lanes with `act`; every
 // lane of the warp calls it. Per bullet in turn: the lanes near it, one after the other, have
 // their search run by the whole warp (contact_search_warp), then take the response themselves.
-__device__ float rubber_contact(const Dev& D, const float2* outlines, int par, uint32_t i, bool act, V3& x, V3& v, float m, V3 load,
+__device__ float rubber_contact(const Dev& D, const Outline* outlines, int par, uint32_t i, bool act, V3& x, V3& v, float m, V3 load,
                                 const VertexForce& vf, bool wet, bool& held, float t, float sub, float now, float dt) {
     const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
     float limit = BIG_F;
@@ -437,7 +468,7 @@ __device__ float rubber_contact(const Dev& D, const float2* outlines, int par, u
     for (uint32_t bi = 0; bi < nbu; bi++) {
         const DBullet b = D.bullets[bi];
         if (b.info.z != 1u) continue;
-        const float2* ol = outlines + bi * NTR_OUTLINE;
+        const Outline& ol = outlines[bi];
         V3 xb = xyz(b.x) - xyz(b.v) * (now - t);
         float closing = length(xyz(b.v) - v);
         const bool near = act && !(length(x - xb) > b.shape.z + vf.reach + 2.0f * closing * dt);
@@ -446,17 +477,9 @@ __device__ float rubber_contact(const Dev& D, const float2* outlines, int par, u
         V3 w = qrot(b.q, qrot(back, xyz(b.l)) / v3(b.shape.y, b.shape.y, b.shape.x));
         for (uint32_t todo = __ballot_sync(full, near); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
-            uint32_t kb = 0, mb = 0;
-            const bool found = contact_search_warp(D, par, src, i, x, v, band, sub, b, xb, back, w, ol, kb, mb);
-            if ((int)lane != src || !found) continue;
-            // The best sample again, with what the response needs.
-            const uint32_t k1 = D.vtri_off[i + 1];
-            const ContactTri tb = contact_tri(D, par, i, kb, k1, x, v, sub, b.shape.w);
-            uint32_t a, c;
-            contact_sample_ac(mb, tb.n, a, c);
             ContactHit hit;
-            float depth_again;
-            contact_sample(ol, tb, a, c, b, xb, back, w, band, depth_again, &hit);
+            const bool found = contact_search_warp(D, par, src, i, x, v, band, sub, b, xb, back, w, ol, hit);
+            if ((int)lane != src || !found) continue;
             const float best = hit.depth;
             const V3 on_b = hit.on_b, gap = hit.gap, nrm = hit.nrm, rel = hit.rel;
             const float share = hit.share;
@@ -570,8 +593,10 @@ __device__ __forceinline__ void mem_substep_body(const Dev& D, const CT& C, uint
     // The contact with the bullets, with every lane of the warp (rubber_contact shares a
     // vertex's search among them), then the rest of the vertex's substep.
     // The bullets' outlines, which every contact sample walks, in shared memory.
-    __shared__ float2 s_outline[NTR_MAX_SHOTS * NTR_OUTLINE];
-    for (uint32_t j = threadIdx.x; j < U->mem[3] * NTR_OUTLINE && j < NTR_MAX_SHOTS * NTR_OUTLINE; j += blockDim.x) s_outline[j] = D.outlines[j];
+    __shared__ Outline s_outline[NTR_MAX_SHOTS];
+    const uint32_t n_seg = min(U->mem[3], (uint32_t)NTR_MAX_SHOTS) * OUTLINE_SEGS;
+    for (uint32_t j = threadIdx.x; j < n_seg; j += blockDim.x)
+        outline_segment(s_outline[j / OUTLINE_SEGS], D.outlines + j / OUTLINE_SEGS * NTR_OUTLINE, j % OUTLINE_SEGS);
     __syncthreads();
     const float lim_c = rubber_contact(D, s_outline, par, i, act, c_x, c_v, c_m, c_f, c_vf, c_ow, c_held, t_sub, sub, now, dt);
     if (act) {

@@ -95,27 +95,6 @@ __device__ __forceinline__ A warp_tree64x2(const SolveLane& L, uint32_t lane, A 
     return s;
 }
 
-// a / b correctly rounded, from y = 1 / b correctly rounded: one step brings a * y within an ulp
-// of the quotient, the second rounds it correctly (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990, theorem on
-// q + r y). It holds while no product or remainder underflows or overflows: 2^-80 <= |a| <= 2^80
-// with 2^-20 <= b <= 2^40 (`quick` says b is; 4e8 random operands, none different from a / b).
-// Zero keeps its sign (b > 0); anything else divides, in a call, which the compiler does not run
-// ahead of its condition: the division takes its long way for a zero numerator, which every warp at
-// the water's surface has (300 cycles a half-sweep beside the rest's 100).
-__device__ __noinline__ float solve_div_any(float a, float b) { return a / b; }
-__device__ __forceinline__ float solve_div(float a, float b, float y, bool quick) {
-    const float m = fabsf(a);
-    const bool fine = quick && m >= 0x1p-80f && m <= 0x1p80f;
-    float q = a * y;
-    float e = __fmaf_rn(-q, b, a);
-    q = __fmaf_rn(e, y, q);
-    e = __fmaf_rn(-q, b, a);
-    q = fine ? __fmaf_rn(e, y, q) : a;
-    if (!fine && !(quick && a == 0.0f)) q = solve_div_any(a, b);
-    return q;
-}
-
 // The padded array of a block: cell (x, y, z), each -1 to 4, at (x + 1) * SOLVE_PX + (y + 1) *
 // SOLVE_PY + z + 1. With these strides the 32 cells of a colour, and their neighbours on one side,
 // fall in 32 banks.
@@ -176,10 +155,10 @@ __device__ __forceinline__ void sts_f(uint32_t a, float v) { asm volatile("st.sh
 // warp. zl: the warp's padded array, -0 around the block: adding it leaves a sum as it is, its sign
 // of zero too. The cells of one colour do not touch each other, so the order in which a half-sweep
 // visits them does not matter. In the first half-sweep every neighbour is still +0.
-__device__ __forceinline__ void warp_precondition(uint32_t zl, const SolveLane& L, SolveCells& C, bool quick) {
+__device__ __forceinline__ void warp_precondition(uint32_t zl, const SolveLane& L, SolveCells& C) {
     const bool w0 = C.water(0), w1 = C.water(1);
     sts_f(zl + 4u * L.at[1], w1 ? 0.0f : -0.0f);
-    float z = solve_div((C.mask & 4u) ? C.r[0] + 0.0f : C.r[0], C.dg[0], C.iv[0], quick);
+    float z = div_by((C.mask & 4u) ? C.r[0] + 0.0f : C.r[0], C.dg[0], C.iv[0]);
     C.z[0] = z;
     sts_f(zl + 4u * L.at[0], w0 ? z : -0.0f);
     __syncwarp();
@@ -187,7 +166,7 @@ __device__ __forceinline__ void warp_precondition(uint32_t zl, const SolveLane& 
         const uint32_t n = zl + 4u * L.at[k];
         const float a = lds_f(n - 4u * SOLVE_PX), b = lds_f(n + 4u * SOLVE_PX), c = lds_f(n - 4u * SOLVE_PY), d = lds_f(n + 4u * SOLVE_PY);
         const float e = lds_f(n - 4u), f = lds_f(n + 4u);
-        z = solve_div(((((((C.r[k] + a) + b) + c) + d) + e) + f), C.dg[k], C.iv[k], quick);
+        z = div_by(((((((C.r[k] + a) + b) + c) + d) + e) + f), C.dg[k], C.iv[k]);
         sts_f(n, (k == 0 ? w0 : w1) ? z : -0.0f);
         C.z[k] = z;
         __syncwarp();
@@ -351,7 +330,6 @@ __device__ __forceinline__ void solve_body(const Dev& D, uint32_t c, uint32_t G,
     const float rho = U->fluid[0];
     const float cs = U->gravity[3] * dt;
     const float kc = hh * hh / (cs * cs);
-    const bool quick = kc >= 0x1p-20f && kc <= 0x1p39f;  // solve_div's range of diagonals: kc to kc + 6
     // Read before the first barrier: thread 0 of CTA 0 writes them back at the end. alpha keeps the last
     // step's value when the solver does not run, as the reference's state does.
     uint32_t iters_max = st->s.iters_max, unconverged = st->s.unconverged;
@@ -479,7 +457,7 @@ __device__ __forceinline__ void solve_body(const Dev& D, uint32_t c, uint32_t G,
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 2; k++) C.dg[k] = s_diag[C.faces(k)], C.iv[k] = s_inv[C.faces(k)];
-        warp_precondition(zl, L, C, quick);
+        warp_precondition(zl, L, C);
         for (int k = 0; k < 2; k++)
             if (C.water(k)) *cfp(D, F_Z, b * 64u + L.li[k]) = C.z[k];
         A sz = warp_tree64(L, M::prod(bq[0], bq[0]), M::prod(bq[1], bq[1]));
@@ -531,7 +509,7 @@ __device__ __forceinline__ void solve_body(const Dev& D, uint32_t c, uint32_t G,
             C.p[k] = C.p[k] + a * C.d[k];
             C.r[k] = C.r[k] - a * C.q[k];
         }
-        warp_precondition(zl, L, C, quick);
+        warp_precondition(zl, L, C);
 #pragma unroll
         for (int k = 0; k < 2; k++)
             if (C.water(k)) *cfp(D, F_Z, b * 64u + L.li[k]) = C.z[k];
