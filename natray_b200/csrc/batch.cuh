@@ -25,7 +25,7 @@
 namespace ntr {
 
 // The kinds of per-scene grids a step's launches use (enqueue_step's grid expressions).
-enum GridKind { GK_ONE, GK_CELL, GK_WORDS, GK_MARK, GK_SCAN, GK_TILES, GK_RSCAN, GK_BOUNDS, GK_BLK, GK_SHOTS, GK_PATCH,
+enum GridKind { GK_ONE, GK_CELL, GK_MARK, GK_SCAN, GK_TILES, GK_RSCAN, GK_BOUNDS, GK_BLK, GK_SHOTS, GK_PATCH,
                 GK_VERT, GK_VERT4, GK_TRI, GK_COUNT };
 
 // A scene's parameters for a batch call (Sim::run sets the same before a one-scene call).
@@ -323,7 +323,6 @@ static void scene_grids(const Sim& S, uint32_t g[GK_COUNT]) {
     const Grids gr = launch_grids(S);
     g[GK_ONE] = 1;
     g[GK_CELL] = gr.cell;
-    g[GK_WORDS] = std::max((D.nwords + 255) / 256, 1u);
     g[GK_MARK] = (uint32_t)(((uint64_t)warp_round(D.Np) + warp_round(D.cap_blocks) + warp_round(D.Nv) + 255) / 256);
     g[GK_SCAN] = D.scan_ctas;
     g[GK_TILES] = D.n_tiles;
@@ -368,10 +367,8 @@ static uint64_t enqueue_step_multi(Batch& B, uint32_t n_jobs, const uint32_t* to
     fork(0, a);
     LM(k_clear_acc_m, GK_CELL, 256, a);
     LM(k_spray_update_m, GK_CELL, 256, a);  // beside the sort, as in enqueue_step
-    LM(k_clear_mask_m, GK_WORDS, 256, s);
     LM(k_mark_m, GK_MARK, 256, s);
-    LM(k_scan_words_a_m, GK_SCAN, SCAN_T, s);
-    LM(k_scan_words_b_m, GK_SCAN, SCAN_T, s);
+    LM(k_scan_words_m, GK_SCAN, SCAN_T, s);
     cudaEventRecord(B.ev_fork[1], s);
     cudaStreamWaitEvent(a, B.ev_fork[1], 0);
     LM(k_mem_splat_m, GK_VERT, 256, a);
@@ -387,14 +384,9 @@ static uint64_t enqueue_step_multi(Batch& B, uint32_t n_jobs, const uint32_t* to
     join(0, a);
     LM(k_gather_prep_m, GK_CELL, 256, s);
     LM(k_air_fill_m, GK_CELL, 256, s);
-    LM(k_bullet_prep_m, GK_SHOTS, 32, s);
-    if (tot[GK_PATCH]) k_bullet_patch_m<<<dim3(tot[GK_PATCH], max_shots), BULLET_PW * 32, 0, s>>>(M(GK_PATCH));
+    if (tot[GK_PATCH]) k_bullet_m<<<dim3(tot[GK_PATCH], max_shots), BULLET_PW * 32, 0, s>>>(M(GK_PATCH));
     nl++;
-    if (prof) prof->mark("k_bullet_patch_m", s);
-    LM(k_bullet_finish_m, GK_SHOTS, 256, s);
-    LM(k_bullet_apply_m, GK_CELL, 256, s);
-    // Every scene's grid barrier counter starts from zero (k_solve_batch keeps one per scene).
-    LM(k_solve_reset_m, GK_ONE, 32, s);
+    if (prof) prof->mark("k_bullet_m", s);
     // Every scene needs a CTA of the joint solve.
     const uint32_t solve_ctas = B.tune.solve_ctas ? std::min(B.ctas, std::max(B.tune.solve_ctas, n_jobs)) : B.ctas;
     nl += enqueue_solve(S0, s, B.d_jobs, n_jobs, fp64, prof, solve_ctas, SOLVE_DYN);

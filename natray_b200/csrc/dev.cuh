@@ -86,14 +86,14 @@ struct DevState {
     ntr_state s;
     double rz, alpha, beta, b_norm, r_norm;
     uint32_t solver_on;
-    uint32_t ticket[4];  // arrival counters of the last-block reductions
+    uint32_t ticket[4];  // per bullet: its CTAs that are done (k_bullet)
     uint32_t nbrk;       // break-ups of this step
     uint32_t err;        // bit 0: a bounded grid barrier gave up
     uint32_t bar_count;  // grid barrier of the persistent solver: arrivals (reset per launch)
-    uint32_t iters_prev;  // the last solve's iterations, kept for a joint solve's split (k_solve_reset_m)
+    uint32_t iters_prev;  // the last solve's iterations, kept for a joint solve's split
     // The next block P2G (0) and G2P (1) hand out in a one-scene launch, zeroed by k_begin_step.
     uint32_t next_block[2];
-    uint32_t pad;
+    uint32_t pushed;  // a bullet pushed on the water in this step (zeroed by k_begin_step)
     // The step's work, for its algorithmic bytes: this step's water and free-gas cells (counted
     // by k_project), and totals since ntr_sim_work last cleared them (added by the step's last
     // kernel): NTR_WORK_STEPS .. NTR_WORK_SPRAY of include/natray.h.
@@ -120,7 +120,7 @@ struct Dev {
     uint32_t* mask[2];
     uint32_t* prefix[2];
     uint32_t* block_list[2];
-    uint32_t* cta_sum;
+    unsigned long long* cta_sum;  // per CTA of the bitmask's scan: the step, and below it its words' bits
     uint32_t *pslot, *key, *key_alt, *val_alt, *key_sorted, *sorted, *hist;
     uint32_t* hist2;  // the sort's second histogram (pass 1's, counted by pass 0's scatter)
     uint32_t *block_start, *block_nb, *block_active;
@@ -143,7 +143,6 @@ struct Dev {
     const float2* outlines;
     DSection* sections;
     int32_t* bullet_hit;
-    float4* bullet_prep;   // per bullet 4 float4: state and pressure ahead, wetted side, impulses
     float4* bullet_patch;  // per bullet and patch 4 float4: force, torque, cavity share
     float4* pose_log;
     float4* spray;  // 3 float4 per slot: pos + r, vel + weight, air

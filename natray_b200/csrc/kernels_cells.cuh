@@ -325,31 +325,14 @@ __global__ void k_air_fill_m(Multi M) {
     air_fill_body(sD, c);
 }
 
-// ---- bullet_apply, bullet.wgsl:385-393 ---------------------------------------------------------------
-template <class CT>
-__device__ __forceinline__ void bullet_apply_body(const Dev& D, const CT& C) {
-    const DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    CELL_LOOP(D, st) {
-#pragma unroll
-        for (uint32_t d = 0; d < 3; d++) {
-            int32_t du = accv(D, A_BU + d, cell);
-            if (du != 0) *cfp(D, F_U + d, cell) = cfv(D, F_U + d, cell) + from_fp(du, FP_M);
-        }
-    }
-}
-// A one-scene step's: CTA 0 also starts the pressure solve's grid barrier counter from zero
-// (one graph node fewer than a memset; a many-scene step has k_solve_reset_m).
-__global__ void k_bullet_apply(Dev D) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) D.st->bar_count = 0u;
-    bullet_apply_body(D, HwCta{});
-}
-__global__ void k_bullet_apply_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (sD.st->parked) return;
-    bullet_apply_body(sD, c);
+// The velocity of face d of `cell` with the bullets' push on it (bullet_apply, bullet.wgsl:385-393),
+// as the pressure solve and the projection read it; the projection leaves it in F_U. `pushed`: whether
+// a bullet pushed on the water in this step at all (DevState::pushed).
+__device__ __forceinline__ float face_pushed(const Dev& D, uint32_t d, uint32_t cell, bool pushed) {
+    const float u = cfv(D, F_U + d, cell);
+    if (!pushed) return u;
+    const int32_t du = accv(D, A_BU + d, cell);
+    return du != 0 ? u + from_fp(du, FP_M) : u;
 }
 
 // ---- the pressure solve -----------------------------------------------------------------------------
@@ -376,6 +359,7 @@ __device__ __forceinline__ void project_body(const Dev& D, const CT& C) {
     if (st->s.dt_ns == 0) return;
     const Grid g = grid_of(D, cur_of(st));
     const float k = dt_of(st) / (D.U->fluid[0] * g.h);
+    const bool pushed = st->pushed != 0u;
     __shared__ uint32_t s_cnt[2];
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
     __syncthreads();
@@ -388,7 +372,7 @@ __device__ __forceinline__ void project_body(const Dev& D, const CT& C) {
         for (uint32_t d = 0; d < 3; d++) {
             uint32_t nb = neighbour(g, cell, ed(d, -1));
             float nt = cell_type(D, nb);
-            float u = bounded(cfv(D, F_U + d, cell), ty, nt);
+            float u = bounded(face_pushed(D, d, cell, pushed), ty, nt);
             if (ty != SOLID_T && nt != SOLID_T && (ty == WATER_T || nt == WATER_T)) u -= k * (pressure_of(D, cell) - pressure_of(D, nb));
             *cfp(D, F_U + d, cell) = u;
         }
@@ -604,15 +588,13 @@ __device__ __forceinline__ float2 sample_grid(const Dev& D, const Grid& g, V3 x,
 __device__ __forceinline__ float wsel(V3 w, int i) { return i == 0 ? w.x : (i == 1 ? w.y : w.z); }
 
 // The sums of the lanes' `vx` and `vy` where `present`, added in lane order, which is the order
-// of the single-thread stencil loops (a, b, c). Every lane gets them.
+// of the single-thread stencil loops (a, b, c). Every lane gets them. An absent lane gives -0, which
+// leaves a sum as it is.
 __device__ __forceinline__ float2 fold27(bool present, float vx, float vy) {
-    const uint32_t pm = __ballot_sync(0xffffffffu, present);
+    const float px = present ? vx : -0.0f, py = present ? vy : -0.0f;
     float sx = 0.0f, sy = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 27; c++) {
-        const float a = __shfl_sync(0xffffffffu, vx, c), b = __shfl_sync(0xffffffffu, vy, c);
-        if ((pm >> c) & 1u) sx = sx + a, sy = sy + b;
-    }
+    for (int c = 0; c < 27; c++) sx = sx + __shfl_sync(0xffffffffu, px, c), sy = sy + __shfl_sync(0xffffffffu, py, c);
     return make_float2(sx, sy);
 }
 

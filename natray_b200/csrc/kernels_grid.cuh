@@ -15,6 +15,9 @@ template <class CT>
 __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
     if (threadIdx.x != 0 || C.x() != 0) return;
     D.st->next_block[0] = D.st->next_block[1] = 0u;
+    D.st->pushed = 0u;
+    D.st->bar_count = 0u;  // the pressure solve's grid barrier
+    D.st->iters_prev = D.st->s.solve_iters;  // for a joint solve's split: every CTA must compute the same one
     const ntr_gpu_params* U = D.U;
     ntr_state& s = D.st->s;
     if (D.st->step_budget == 0u) {  // a batch scene that has taken its steps of the call
@@ -73,9 +76,9 @@ __global__ void k_begin_step_m(Multi M) {
     begin_step_body(sD, c);
 }
 
-// ---- clear: the last step's transfer sums, and this step's bitmask ----------------------------
+// ---- clear: the last step's transfer sums ------------------------------------------------------
 // Fields 0..7 of the sums are written whole by k_p2g_gather and A_N by k_p2g; the rest
-// accumulate atomically and start from zero. The two clears run on different streams.
+// accumulate atomically and start from zero.
 template <class CT>
 __device__ __forceinline__ void clear_acc_body(const Dev& D, const CT& C) {
     const DevState* st = D.st;
@@ -98,29 +101,21 @@ __global__ void k_clear_acc_m(Multi M) {
     clear_acc_body(sD, c);
 }
 
-template <class CT>
-__device__ __forceinline__ void clear_mask_body(const Dev& D, const CT& C) {
-    const DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    uint32_t* m = D.mask[cur_of(st)];
-    for (size_t w = (size_t)C.x() * blockDim.x + threadIdx.x; w < D.nwords; w += (size_t)C.nx() * blockDim.x) m[w] = 0u;
+// Sets `bits` of the bitmask's word `word` of the lanes where bits are not zero: one atomicOr per
+// distinct word in the warp, with the bits of all its lanes. All 32 lanes call it.
+__device__ __forceinline__ void set_word_bits(uint32_t* mask, uint32_t word, uint32_t bits) {
+    if (!__any_sync(0xffffffffu, bits != 0u)) return;
+    const uint32_t key = bits ? word : NONE;
+    const uint32_t peers = __match_any_sync(0xffffffffu, key);
+    const uint32_t all = __reduce_or_sync(peers, bits);
+    if (bits && (__ffs(peers) - 1) == (int)(threadIdx.x & 31u)) atomicOr(mask + word, all);
 }
-__global__ void k_clear_mask(Dev D) { clear_mask_body(D, HwCta{}); }
-__global__ void k_clear_mask_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (sD.st->parked) return;
-    clear_mask_body(sD, c);
-}
-
-// Sets the bits of the blocks `slot` of the lanes where `valid`: one atomicOr per distinct
-// word of the bitmask in the warp, with the bits of all its lanes. All 32 lanes call it.
-__device__ __forceinline__ void set_block_bits(uint32_t* mask, uint32_t slot, bool valid) {
-    const uint32_t word = valid ? slot >> 5 : NONE;
-    const uint32_t peers = __match_any_sync(0xffffffffu, word);
-    const uint32_t bits = __reduce_or_sync(peers, valid ? 1u << (slot & 31u) : 0u);
-    if (valid && (__ffs(peers) - 1) == (int)(threadIdx.x & 31u)) atomicOr(mask + word, bits);
+// Sets the bits of `n` blocks in a row along z from `slot` (n <= 32; none where n is 0). Slots run
+// along z, so a row's bits are one word's, or for a row over a word's end two words'.
+__device__ __forceinline__ void set_block_row(uint32_t* mask, uint32_t slot, uint32_t n) {
+    const uint64_t bits = ((1ull << n) - 1ull) << (slot & 31u);
+    set_word_bits(mask, slot >> 5, (uint32_t)bits);
+    set_word_bits(mask, (slot >> 5) + 1u, (uint32_t)(bits >> 32));
 }
 
 __host__ __device__ __forceinline__ uint32_t warp_round(uint32_t n) { return (n + 31u) & ~31u; }
@@ -157,17 +152,20 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
             I3 ob = shr2(c);
             D.pslot[i] = (alive && in_bd(g, ob)) ? block_slot(g, ob) : NONE;
         }
-        for (int k = 0; k < 8; k++) {
-            I3 b = {lo.x + (k & 1), lo.y + ((k >> 1) & 1), lo.z + ((k >> 2) & 1)};
-            bool valid = alive && b.x <= hi.x && b.y <= hi.y && b.z <= hi.z;
-            set_block_bits(mask, valid ? block_slot(g, b) : 0u, valid);
+        // A row of one or two along z for each of up to four (x, y): the bits of a warp's rows are
+        // merged per word before they go out, four merges instead of one for each of eight blocks.
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const I3 b = {lo.x + (k & 1), lo.y + (k >> 1), lo.z};
+            const bool valid = alive && b.x <= hi.x && b.y <= hi.y;
+            set_block_row(mask, valid ? block_slot(g, b) : 0u, valid ? (uint32_t)(hi.z - lo.z + 1) : 0u);
         }
         return;
     }
     uint32_t j = i - np_w;
     if (j < nb_w) {
         const bool valid = j < n_prev && D.block_active[j] != 0u;
-        set_block_bits(mask, valid ? D.block_list[cur ^ 1][j] : 0u, valid);
+        set_block_row(mask, valid ? D.block_list[cur ^ 1][j] : 0u, valid ? 1u : 0u);
         return;
     }
     j -= nb_w;
@@ -186,10 +184,10 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
         }
     }
     if (!__any_sync(0xffffffffu, dry)) return;
-    for (int k = 0; k < 27; k++) {
-        I3 b = {lo.x + k / 9, lo.y + (k / 3) % 3, lo.z + k % 3};
-        bool valid = dry && b.x <= hi.x && b.y <= hi.y && b.z <= hi.z;
-        set_block_bits(mask, valid ? block_slot(g, b) : 0u, valid);
+    for (int k = 0; k < 9; k++) {
+        const I3 b = {lo.x + k / 3, lo.y + k % 3, lo.z};
+        const bool valid = dry && b.x <= hi.x && b.y <= hi.y;
+        set_block_row(mask, valid ? block_slot(g, b) : 0u, valid ? (uint32_t)(hi.z - lo.z + 1) : 0u);
     }
 }
 __global__ void k_mark(Dev D) { mark_body(D, HwCta{}); }
@@ -204,51 +202,20 @@ __global__ void k_mark_m(Multi M) {
 // ---- compaction of the bitmask: blocks numbered in ascending slot order ----------------------
 constexpr int SCAN_T = 256, SCAN_W = 8;  // 2048 words per CTA
 
+// One launch: a CTA counts its words' bits, leaves the count for the CTAs after it and takes the
+// counts of those before it as they come (each with the number of its step beside it, in a word
+// written whole; a CTA waits only for CTAs that were launched before it, at most D.bar_spins polls).
+// Two launches before, the counts and then the rest: the second one waited 4 us for the first.
 template <class CT>
-__device__ __forceinline__ void scan_words_a_body(const Dev& D, const CT& C) {
-    const DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    const uint32_t* m = D.mask[cur_of(st)];
-    uint32_t base = C.x() * SCAN_T * SCAN_W;
-    uint32_t s = 0;
-    for (int k = 0; k < SCAN_W; k++) {
-        uint32_t w = base + k * SCAN_T + threadIdx.x;
-        if (w < D.nwords) s += __popc(m[w]);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __shared__ uint32_t ws[SCAN_T / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int k = 0; k < SCAN_T / 32; k++) t += ws[k];
-        D.cta_sum[C.x()] = t;
-    }
-}
-__global__ void __launch_bounds__(SCAN_T) k_scan_words_a(Dev D) { scan_words_a_body(D, HwCta{}); }
-__global__ void __launch_bounds__(SCAN_T) k_scan_words_a_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (sD.st->parked) return;
-    scan_words_a_body(sD, c);
-}
-
-template <class CT>
-__device__ __forceinline__ void scan_words_b_body(const Dev& D, const CT& C) {
+__device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
     DevState* st = D.st;
     if (st->s.dt_ns == 0) return;
     const int cur = cur_of(st);
     const uint32_t* m = D.mask[cur];
     uint32_t* prefix = D.prefix[cur];
     uint32_t* list = D.block_list[cur];
+    const unsigned long long tag = ((unsigned long long)st->s.step << 1) | 1ull;  // above 31 bits of count; a new state's words, zero, match none
     __shared__ uint32_t s_base, ws[SCAN_T / 32];
-    if (threadIdx.x < 32) {
-        uint32_t t = 0;
-        for (uint32_t k = threadIdx.x; k < C.x(); k += 32) t += D.cta_sum[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        if (threadIdx.x == 0) s_base = t;
-    }
     // Each thread owns SCAN_W consecutive words (two 16-byte loads where all are in range).
     static_assert(SCAN_W == 8, "two uint4 per thread");
     uint32_t w0 = C.x() * SCAN_T * SCAN_W + threadIdx.x * SCAN_W;
@@ -269,6 +236,26 @@ __device__ __forceinline__ void scan_words_b_body(const Dev& D, const CT& C) {
         if (lane >= (uint32_t)o) inc += v;
     }
     if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t t = 0;
+            for (int k = 0; k < SCAN_T / 32; k++) t += ws[k];
+            *(volatile unsigned long long*)(D.cta_sum + C.x()) = (tag << 31) | t;
+        }
+        uint32_t t = 0;
+        for (uint32_t k = lane; k < C.x(); k += 32) {
+            unsigned long long v;
+            for (uint32_t spins = 0; ((v = *(volatile const unsigned long long*)(D.cta_sum + k)) >> 31) != tag;)
+                if (++spins > D.bar_spins) {
+                    atomicOr(&st->err, 1u);
+                    break;
+                }
+            t += (uint32_t)v & 0x7fffffffu;
+        }
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) s_base = t;
+    }
     __syncthreads();
     uint32_t wbase = 0;
     for (uint32_t k = 0; k < warp; k++) wbase += ws[k];
@@ -293,13 +280,13 @@ __device__ __forceinline__ void scan_words_b_body(const Dev& D, const CT& C) {
         if (run > cap) st->s.overflow = 1u;
     }
 }
-__global__ void __launch_bounds__(SCAN_T) k_scan_words_b(Dev D) { scan_words_b_body(D, HwCta{}); }
-__global__ void __launch_bounds__(SCAN_T) k_scan_words_b_m(Multi M) {
+__global__ void __launch_bounds__(SCAN_T) k_scan_words(Dev D) { scan_words_body(D, HwCta{}); }
+__global__ void __launch_bounds__(SCAN_T) k_scan_words_m(Multi M) {
     __shared__ Dev sD;
     __shared__ Cta c;
     multi_cta(M, sD, c);
     if (sD.st->parked) return;
-    scan_words_b_body(sD, c);
+    scan_words_body(sD, c);
 }
 
 // ---- keys: each live particle's block index ---------------------------------------------------
@@ -866,6 +853,10 @@ __device__ __forceinline__ void gather_prep_body(const Dev& D, const CT& C) {
         for (int f = 0; f < 8; f++) D.acc[(size_t)f * D.cap_cells + cell] = s8[f];
         grid_prep_cell(D, g, knot, kr, dt, grav, cell, s8);
     }
+    // The last step's block bitmask, which the air's carry was the last to read, is the next step's:
+    // its blocks' words are cleared here (a launch over the whole domain's bitmask before).
+    const int old = cur_of(st) ^ 1;
+    for (uint32_t b = C.x() * blockDim.x + threadIdx.x; b < st->s.n_blocks_prev; b += C.nx() * blockDim.x) D.mask[old][D.block_list[old][b] >> 5] = 0u;
 }
 __global__ void k_gather_prep(Dev D) { gather_prep_body(D, HwCta{}); }
 __global__ void k_gather_prep_m(Multi M) {

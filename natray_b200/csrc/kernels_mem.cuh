@@ -640,8 +640,8 @@ __device__ __forceinline__ float cp_patch(float s) {
 
 __device__ __forceinline__ float section_r2(const DSection& s, float t) { return s.c.x + s.b.w * mx(t - s.a.w, 0.0f); }
 
-// sample_pressure by a warp.
-__device__ __forceinline__ float2 warp_sample_pressure(const Dev& D, const Grid& g, V3 x, bool gas_only, int lane) {
+// The water pressure ahead of a bullet, at x (grid units, less a half), by a warp.
+__device__ __forceinline__ float2 warp_pressure_ahead(const Dev& D, const Grid& g, V3 x, int lane) {
     I3 base = vi(vfloor(x - 0.5f));
     V3 fx = x - vf(base);
     V3 wx = axis_weights(fx.x), wy = axis_weights(fx.y), wz = axis_weights(fx.z);
@@ -650,13 +650,10 @@ __device__ __forceinline__ float2 warp_sample_pressure(const Dev& D, const Grid&
     float wp = 0.0f, w = 0.0f;
     if (lane < 27) {
         const uint32_t cell = cell_at(g, base + I3{a, b, c});
-        if (cell != NONE) {
-            const float ty = cfv(D, F_TYPE, cell);
-            if (!(ty == SOLID_T || (gas_only && ty == WATER_T))) {
-                present = true;
-                w = wsel(wx, a) * wsel(wy, b) * wsel(wz, c);
-                wp = w * cfv(D, F_P, cell);
-            }
+        if (cell != NONE && cfv(D, F_TYPE, cell) != SOLID_T) {
+            present = true;
+            w = wsel(wx, a) * wsel(wy, b) * wsel(wz, c);
+            wp = w * cfv(D, F_P, cell);
         }
     }
     return fold27(present, wp, w);
@@ -664,7 +661,7 @@ __device__ __forceinline__ float2 warp_sample_pressure(const Dev& D, const Grid&
 
 // The five samples of a bullet patch at X (grid units) by a warp: the water velocity of the
 // three face lattices (warp_sample_grid with F_U + d, a_wt(d)), the fill (F_TYPE, A_WC at
-// X - 0.5) and the gas pressure (warp_sample_pressure at X - 0.5, gas only, the fill's stencil).
+// X - 0.5) and the gas pressure (at X - 0.5, of cells neither solid nor water, the fill's stencil).
 // Each lane's four cell lookups and then all their loads go out together, instead of one
 // sample's dependent chain after another's; the folds are the same, in the same order.
 __device__ __forceinline__ void warp_patch_samples(const Dev& D, const Grid& g, V3 X, int lane, float2 (&s)[4], float2& gs) {
@@ -720,6 +717,7 @@ __device__ __forceinline__ void warp_push_water(const Dev& D, const Grid& g, V3 
     const int a = lane / 9, b = (lane / 3) % 3, c = lane % 3;
     const uint32_t cell = cell_at(g, base + I3{a, b, c});
     if (cell == NONE || accv(D, a_wt(d), cell) <= 0) return;
+    D.st->pushed = 1u;
     atomicAdd(accp(D, A_BU + d, cell), to_fp(k * wsel(wx, a) * wsel(wy, b) * wsel(wz, c), FP_M));
 }
 
@@ -740,166 +738,27 @@ __device__ __forceinline__ bool warp_in_cavity(const Dev& D, float hh, uint32_t 
     return __any_sync(0xffffffffu, in);
 }
 
-// The bullets' step (bullet.wgsl:186-383) in three launches:
-//   k_bullet_prep, a warp per bullet: whether it flies this step, the water pressure ahead of
-//     it, the membrane's contact sums (taken and cleared), into `bullet_prep`;
-//   k_bullet_patch, a warp per surface patch: the patch's loads and its push on the water, into
-//     `bullet_patch`;
-//   k_bullet_finish, a CTA per bullet: the patches summed in the reference's order (lane l of
-//     256 takes patches l, l + 256, l + 512 in turn, then a 256-wide tree), the rigid body, the
-//     cavity sections.
-template <class CT>
-__device__ __forceinline__ void bullet_prep_body(const Dev& D, const CT& C) {
+// The bullets' step (bullet.wgsl:186-383) in one launch, a warp per surface patch (<= 576 a bullet):
+// the water pressure ahead of the bullet and the patch's loads and push on the water, into
+// `bullet_patch`; then, in the CTA that finishes last of a bullet's (a counter taken after a fence;
+// no CTA waits for another), the patches summed in the reference's order (lane l of 256 takes
+// patches l, l + 256, l + 512 in turn, then a 256-wide tree), the membrane's contact sums taken and
+// cleared, the rigid body, the cavity sections. Three launches before (the pressure ahead, the
+// patches, the sum): beside their work each cost about 4 us of the step.
+// A bullet's patches summed, its body moved, its sections: by a CTA of 256 threads, all patches done.
+__device__ __forceinline__ void bullet_finish(const Dev& D, const Grid& g, uint32_t bi, const DBullet& b, int32_t* hit) {
     DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    const uint32_t bi = C.x();
-    // A scene without bullets still launches one CTA; it has nothing to do (and the patch and
-    // finish kernels skip a bullet whose prep flag is not set).
-    if (bi >= D.U->mem[3]) {
-        if (threadIdx.x == 0) D.bullet_prep[bi * 4].x = 0.0f;
-        return;
-    }
-    const int lane = (int)threadIdx.x;
-    const Grid g = grid_of(D, cur_of(st));
-    const DBullet b = D.bullets[bi];
-    const float hh = g.h;
-    int32_t* hit = D.bullet_hit + bi * NTR_HIT_FIELDS;
-    uint32_t state = b.info.z;
-    if (state == 0u && st->s.t_ns - st->s.dt_ns >= b.info.x) state = 1u;
-    // The wetted-side sums always, the impulses only when the bullet flies this step.
-    int32_t hv = 0;
-    if (lane < NTR_HIT_FIELDS) hv = ((uint32_t)lane >= 6u || state == 1u) ? atomicExch(hit + lane, 0) : 0;
-    int32_t h[NTR_HIT_FIELDS];
-#pragma unroll
-    for (int c = 0; c < NTR_HIT_FIELDS; c++) h[c] = __shfl_sync(0xffffffffu, hv, c);
-    V3 ahead = xyz(b.x) + normalize(xyz(b.v) + 1e-9f) * (b.shape.z + 3.0f * hh);
-    const V3 xa = (ahead - g.org) / hh - 0.5f;
-    const float2 s = warp_sample_pressure(D, g, xa, false, lane);
-    if (lane != 0) return;
-    const float pf = s.y > 1e-6f ? s.x / s.y : 0.0f;
-    V3 sn, sx;
-    for (int c = 0; c < 3; c++) {
-        sn[c] = from_fp(h[6 + c], FP_A);
-        sx[c] = from_fp(h[9 + c], FP_X);
-    }
-    float sa = from_fp(h[12], FP_A);
-    float4 side = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (sa > 0.0f && length(sn) > 0.0f) {
-        V3 n = normalize(sn);
-        side = make_float4(n.x, n.y, n.z, dot(sx, n) / sa * 1e-3f);
-    }
-    float4* o = D.bullet_prep + bi * 4;
-    o[0] = make_float4(__uint_as_float(state), pf, 0.0f, 0.0f);
-    o[1] = side;
-    o[2] = make_float4(__int_as_float(h[0]), __int_as_float(h[1]), __int_as_float(h[2]), __int_as_float(h[3]));
-    o[3] = make_float4(__int_as_float(h[4]), __int_as_float(h[5]), 0.0f, 0.0f);
-    if (state != 1u) {
-        D.bullets[bi].info.z = state;
-        D.pose_log[(bi * NTR_LOG_CAP + st->s.step % NTR_LOG_CAP) * 3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-}
-__global__ void k_bullet_prep(Dev D) { bullet_prep_body(D, HwCta{}); }
-__global__ void k_bullet_prep_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (sD.st->parked) return;
-    bullet_prep_body(sD, c);
-}
-
-constexpr int BULLET_PW = 8;  // patch warps per CTA
-
-template <class CT>
-__device__ __forceinline__ void bullet_patch_body(const Dev& D, const CT& C) {
-    DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    const uint32_t bi = C.y();
-    const float4 pr = D.bullet_prep[bi * 4];
-    if (__float_as_uint(pr.x) != 1u) return;
-    const DBullet b = D.bullets[bi];
-    const uint32_t k = C.x() * BULLET_PW + (threadIdx.x >> 5);
-    if (k >= b.info.y) return;
-    const int lane = (int)(threadIdx.x & 31u);
-    const Grid g = grid_of(D, cur_of(st));
-    const ntr_gpu_params* U = D.U;
-    const float step = dt_of(st), t_end = now_of(st), hh = g.h;
-    const float pf = pr.y;
-    const float4 side = D.bullet_prep[bi * 4 + 1];
-    V3 lb = qrot(make_float4(-b.q.x, -b.q.y, -b.q.z, b.q.w), xyz(b.l));
-    V3 w = qrot(b.q, lb / v3(b.shape.y, b.shape.y, b.shape.x));
-    const float rho = U->fluid[0];
-    const V3 vhat = normalize(xyz(b.v) + 1e-9f);
-    // The patch's force, torque, push on the water, and share of the wetted face.
-    V3 fp = {0.0f, 0.0f, 0.0f}, tqp = {0.0f, 0.0f, 0.0f}, cenp = {0.0f, 0.0f, 0.0f};
-    float cavxp = 0.0f, cavyp = 0.0f, cenwp = BIG_F;
-    bool has_cav = false;
-    const float4 pp = D.patches[(bi * NTR_MAX_PATCHES + k) * 2], pn = D.patches[(bi * NTR_MAX_PATCHES + k) * 2 + 1];
-    V3 r = qrot(b.q, xyz(pp));
-    V3 p = xyz(b.x) + r;
-    V3 n = qrot(b.q, xyz(pn));
-    float area = pp.w;
-    V3 X = (p - g.org) / hh;
-    float2 sm[4], gs;
-    warp_patch_samples(D, g, X, lane, sm, gs);
-    const float2 s0 = sm[0], s1 = sm[1], s2 = sm[2];
-    V3 uw = {s0.y > 1e-6f ? s0.x / s0.y : 0.0f, s1.y > 1e-6f ? s1.x / s1.y : 0.0f, s2.y > 1e-6f ? s2.x / s2.y : 0.0f};
-    V3 sw = {s0.y, s1.y, s2.y};
-    float fill = clampf_(sm[3].y / 8.0f, 0.0f, 1.0f);
-    if (warp_in_cavity(D, hh, bi, p, t_end - step, lane) || dot(r, xyz(side)) > side.w) fill = 0.0f;
-    float p_gas = gs.y > 1e-6f ? gs.x / gs.y : 0.0f;
-    V3 vp = xyz(b.v) + cross(w, r);
-    V3 rel = vp - uw;
-    float spd = length(rel);
-    float wn = dot(rel, n);
-    float q = 0.5f * rho * spd * spd;
-    float p_water = mx(P_VAPOUR - P_ATM, pf + q * cp_patch(wn / mx(spd, 1e-9f)));
-    V3 fw = -fill * p_water * area * n;
-    V3 rt = rel - wn * n;
-    float rtl = length(rt);
-    if (rtl > 1e-9f) fw = fw - fill * CF_SKIN * 0.5f * rho * rtl * rt * area;
-    fp = fw - (1.0f - fill) * mx(p_gas, P_VAPOUR - P_ATM) * area * n;
-    tqp = cross(r, fp);
-    warp_push_water(D, g, X, 0, -fw.x * step, sw.x, lane);
-    warp_push_water(D, g, X, 1, -fw.y * step, sw.y, lane);
-    warp_push_water(D, g, X, 2, -fw.z * step, sw.z, lane);
-    if (wn > 0.0f && fill > 0.0f) {
-        float face = fill * area * mx(dot(n, vhat), 0.0f);
-        has_cav = true;
-        cavxp = -dot(fw, vhat);
-        cavyp = face;
-        cenp = p * face;
-        cenwp = dot(r, vhat);
-    }
-    if (lane == 0) {
-        float4* o = D.bullet_patch + (bi * NTR_MAX_PATCHES + k) * 4;
-        o[0] = f4(fp, cavxp);
-        o[1] = f4(tqp, cavyp);
-        o[2] = f4(cenp, cenwp);
-        o[3] = make_float4(has_cav ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
-    }
-}
-__global__ void __launch_bounds__(BULLET_PW * 32) k_bullet_patch(Dev D) { bullet_patch_body(D, HwCta{}); }
-__global__ void __launch_bounds__(BULLET_PW * 32) k_bullet_patch_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (sD.st->parked) return;
-    bullet_patch_body(sD, c);
-}
-
-template <class CT>
-__device__ __forceinline__ void bullet_finish_body(const Dev& D, const CT& C) {
-    DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
-    const uint32_t bi = C.x();
-    if (__float_as_uint(D.bullet_prep[bi * 4].x) != 1u) return;
-    const Grid g = grid_of(D, cur_of(st));
     const ntr_gpu_params* U = D.U;
     const uint32_t li = threadIdx.x;
-    const DBullet b = D.bullets[bi];
     const float step = dt_of(st), t_end = now_of(st), hh = g.h;
     const float rho = U->fluid[0];
     const V3 vhat = normalize(xyz(b.v) + 1e-9f);
+    // The membrane's contact sums are this step's: taken and cleared.
+    __shared__ int32_t s_hit[6];
+    if (li < NTR_HIT_FIELDS) {
+        if (li < 6) s_hit[li] = hit[li];
+        hit[li] = 0;
+    }
     __shared__ float4 red_f[256], red_t[256], red_c[256];
     const uint32_t n_patch = b.info.y;
     // Lane l's running sums over patches l, l + 256, l + 512, in that order.
@@ -910,10 +769,10 @@ __device__ __forceinline__ void bullet_finish_body(const Dev& D, const CT& C) {
         const uint32_t k = li + round * 256u;
         if (k < n_patch) {
             const float4* rec = D.bullet_patch + (bi * NTR_MAX_PATCHES + k) * 4;
-            const float4 a = rec[0], t4 = rec[1], c4 = rec[2];
+            const float4 a = __ldcg(rec), t4 = __ldcg(rec + 1), c4 = __ldcg(rec + 2);
             f = f + xyz(a);
             tq = tq + xyz(t4);
-            if (rec[3].x != 0.0f) {
+            if (__ldcg(rec + 3).x != 0.0f) {
                 cavx = cavx + a.w;
                 cavy = cavy + t4.w;
                 V3 cx = v3(cen.x, cen.y, cen.z) + xyz(c4);
@@ -935,12 +794,6 @@ __device__ __forceinline__ void bullet_finish_body(const Dev& D, const CT& C) {
             red_c[li] = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, mn(a.w, o.w));
         }
         __syncthreads();
-    }
-    int32_t s_hit[6];
-    {
-        const float4 h0 = D.bullet_prep[bi * 4 + 2], h1 = D.bullet_prep[bi * 4 + 3];
-        s_hit[0] = __float_as_int(h0.x), s_hit[1] = __float_as_int(h0.y), s_hit[2] = __float_as_int(h0.z);
-        s_hit[3] = __float_as_int(h0.w), s_hit[4] = __float_as_int(h1.x), s_hit[5] = __float_as_int(h1.y);
     }
     const float hand2 = R_HAND * R_HAND * hh * hh;
     // The new velocity and position (every thread; the 27 blocks around it are looked up in
@@ -1037,13 +890,141 @@ __device__ __forceinline__ void bullet_finish_body(const Dev& D, const CT& C) {
         }
     }
 }
-__global__ void __launch_bounds__(256) k_bullet_finish(Dev D) { bullet_finish_body(D, HwCta{}); }
-__global__ void __launch_bounds__(256) k_bullet_finish_m(Multi M) {
+constexpr int BULLET_PW = 8;  // patch warps per CTA
+
+// One surface patch by a warp, at p (and X in grid units), r from the bullet's centre: its loads and
+// its push on the water. pf: the pressure ahead; sm, gs: its samples (warp_patch_samples).
+__device__ __forceinline__ void bullet_patch(const Dev& D, const Grid& g, uint32_t bi, uint32_t k, const DBullet& b, const int32_t* hit, int lane,
+                                             V3 r, V3 p, V3 X, float area, float pf, const float2 (&sm)[4], float2 gs) {
+    const DevState* st = D.st;
+    const ntr_gpu_params* U = D.U;
+    const float step = dt_of(st), t_end = now_of(st), hh = g.h;
+    // The side the rubber wets, from the contact sums of the last step's substeps.
+    int32_t h[7];
+#pragma unroll
+    for (int c = 0; c < 7; c++) h[c] = hit[6 + c];
+    V3 sn, sx;
+    for (int c = 0; c < 3; c++) {
+        sn[c] = from_fp(h[c], FP_A);
+        sx[c] = from_fp(h[3 + c], FP_X);
+    }
+    float sa = from_fp(h[6], FP_A);
+    float4 side = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (sa > 0.0f && length(sn) > 0.0f) {
+        V3 n = normalize(sn);
+        side = make_float4(n.x, n.y, n.z, dot(sx, n) / sa * 1e-3f);
+    }
+    V3 lb = qrot(make_float4(-b.q.x, -b.q.y, -b.q.z, b.q.w), xyz(b.l));
+    V3 w = qrot(b.q, lb / v3(b.shape.y, b.shape.y, b.shape.x));
+    const float rho = U->fluid[0];
+    const V3 vhat = normalize(xyz(b.v) + 1e-9f);
+    // The patch's force, torque, push on the water, and share of the wetted face.
+    V3 fp = {0.0f, 0.0f, 0.0f}, tqp = {0.0f, 0.0f, 0.0f}, cenp = {0.0f, 0.0f, 0.0f};
+    float cavxp = 0.0f, cavyp = 0.0f, cenwp = BIG_F;
+    bool has_cav = false;
+    const V3 n = qrot(b.q, xyz(D.patches[(bi * NTR_MAX_PATCHES + k) * 2 + 1]));
+    const float2 s0 = sm[0], s1 = sm[1], s2 = sm[2];
+    V3 uw = {s0.y > 1e-6f ? s0.x / s0.y : 0.0f, s1.y > 1e-6f ? s1.x / s1.y : 0.0f, s2.y > 1e-6f ? s2.x / s2.y : 0.0f};
+    V3 sw = {s0.y, s1.y, s2.y};
+    float fill = clampf_(sm[3].y / 8.0f, 0.0f, 1.0f);
+    if (warp_in_cavity(D, hh, bi, p, t_end - step, lane) || dot(r, xyz(side)) > side.w) fill = 0.0f;
+    float p_gas = gs.y > 1e-6f ? gs.x / gs.y : 0.0f;
+    V3 vp = xyz(b.v) + cross(w, r);
+    V3 rel = vp - uw;
+    float spd = length(rel);
+    float wn = dot(rel, n);
+    float q = 0.5f * rho * spd * spd;
+    float p_water = mx(P_VAPOUR - P_ATM, pf + q * cp_patch(wn / mx(spd, 1e-9f)));
+    V3 fw = -fill * p_water * area * n;
+    V3 rt = rel - wn * n;
+    float rtl = length(rt);
+    if (rtl > 1e-9f) fw = fw - fill * CF_SKIN * 0.5f * rho * rtl * rt * area;
+    fp = fw - (1.0f - fill) * mx(p_gas, P_VAPOUR - P_ATM) * area * n;
+    tqp = cross(r, fp);
+    warp_push_water(D, g, X, 0, -fw.x * step, sw.x, lane);
+    warp_push_water(D, g, X, 1, -fw.y * step, sw.y, lane);
+    warp_push_water(D, g, X, 2, -fw.z * step, sw.z, lane);
+    if (wn > 0.0f && fill > 0.0f) {
+        float face = fill * area * mx(dot(n, vhat), 0.0f);
+        has_cav = true;
+        cavxp = -dot(fw, vhat);
+        cavyp = face;
+        cenp = p * face;
+        cenwp = dot(r, vhat);
+    }
+    if (lane == 0) {
+        float4* o = D.bullet_patch + (bi * NTR_MAX_PATCHES + k) * 4;
+        o[0] = f4(fp, cavxp);
+        o[1] = f4(tqp, cavyp);
+        o[2] = f4(cenp, cenwp);
+        o[3] = make_float4(has_cav ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+
+template <class CT>
+__device__ __forceinline__ void bullet_body(const Dev& D, const CT& C) {
+    DevState* st = D.st;
+    if (st->s.dt_ns == 0) return;
+    const ntr_gpu_params* U = D.U;
+    const uint32_t bi = C.y();
+    if (bi >= U->mem[3]) return;  // a scene with fewer bullets, or none
+    const DBullet b = D.bullets[bi];
+    int32_t* hit = D.bullet_hit + bi * NTR_HIT_FIELDS;
+    uint32_t state = b.info.z;
+    if (state == 0u && st->s.t_ns - st->s.dt_ns >= b.info.x) state = 1u;
+    if (state != 1u) {
+        // Not flying this step: the wetted-side sums are cleared all the same, the impulses kept.
+        if (C.x() != 0) return;
+        if (threadIdx.x >= 6 && threadIdx.x < NTR_HIT_FIELDS) hit[threadIdx.x] = 0;
+        if (threadIdx.x == 0) {
+            D.bullets[bi].info.z = state;
+            D.pose_log[(bi * NTR_LOG_CAP + st->s.step % NTR_LOG_CAP) * 3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        return;
+    }
+    const uint32_t k = C.x() * BULLET_PW + (threadIdx.x >> 5);
+    const int lane = (int)(threadIdx.x & 31u);
+    const Grid g = grid_of(D, cur_of(st));
+    // The water pressure ahead, once a CTA, by its first warp beside the patches' samples.
+    __shared__ float s_pf;
+    if (threadIdx.x < 32) {
+        const V3 ahead = xyz(b.x) + normalize(xyz(b.v) + 1e-9f) * (b.shape.z + 3.0f * g.h);
+        const float2 ps = warp_pressure_ahead(D, g, (ahead - g.org) / g.h - 0.5f, lane);
+        if (lane == 0) s_pf = ps.y > 1e-6f ? ps.x / ps.y : 0.0f;
+    }
+    float2 sm[4], gs;
+    V3 r = {0.0f, 0.0f, 0.0f}, p = r, X = r;
+    float area = 0.0f;
+    if (k < b.info.y) {
+        const float4 pp = D.patches[(bi * NTR_MAX_PATCHES + k) * 2];
+        r = qrot(b.q, xyz(pp));
+        p = xyz(b.x) + r;
+        X = (p - g.org) / g.h;
+        area = pp.w;
+        warp_patch_samples(D, g, X, lane, sm, gs);
+    }
+    __syncthreads();
+    if (k < b.info.y) bullet_patch(D, g, bi, k, b, hit, lane, r, p, X, area, s_pf, sm, gs);
+    // The CTA that is last of the bullet's.
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&st->ticket[bi], 1u) == C.nx() - 1u;
+        if (s_last) st->ticket[bi] = 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    bullet_finish(D, g, bi, b, hit);
+}
+__global__ void __launch_bounds__(BULLET_PW * 32) k_bullet(Dev D) { bullet_body(D, HwCta{}); }
+__global__ void __launch_bounds__(BULLET_PW * 32) k_bullet_m(Multi M) {
     __shared__ Dev sD;
     __shared__ Cta c;
     multi_cta(M, sD, c);
     if (sD.st->parked) return;
-    bullet_finish_body(sD, c);
+    bullet_body(sD, c);
 }
 
 // The rubber's substep kernels over many scenes: substep i of the step, for the scenes whose

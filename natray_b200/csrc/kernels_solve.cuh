@@ -27,7 +27,7 @@
 //   - a warp with one block keeps all this in registers for the whole solve; with more, in a
 //     record per block (SolveRec), in shared memory while the CTA's blocks fit there and else in
 //     D.wnb;
-//   - the grid barrier is a counter that only grows during the launch (reset before it): the
+//   - the grid barrier is a counter that only grows during the launch (k_begin_step resets it): the
 //     k-th barrier waits for k * (CTAs) arrivals. One atomic per CTA and a poll of the same word.
 //     (Values that carry the number of their exchange and are polled themselves, no counter and no
 //     fence, were slower at every size: 1M particles 108 us against 93, 66k 64 against 51; so were
@@ -330,6 +330,7 @@ __device__ __forceinline__ void solve_body(const Dev& D, uint32_t c, uint32_t G,
     const float rho = U->fluid[0];
     const float cs = U->gravity[3] * dt;
     const float kc = hh * hh / (cs * cs);
+    const bool pushed = st->pushed != 0u;
     // Read before the first barrier: thread 0 of CTA 0 writes them back at the end. alpha keeps the last
     // step's value when the solver does not run, as the reference's state does.
     uint32_t iters_max = st->s.iters_max, unconverged = st->s.unconverged;
@@ -396,14 +397,14 @@ __device__ __forceinline__ void solve_body(const Dev& D, uint32_t c, uint32_t G,
             const float dold = cfv(D, F_D, cell);
             const int32_t src = accv(D, A_SRC, cell);
 #pragma unroll
-            for (int d = 0; d < 3; d++) uc[d] = cfv(D, F_U + d, cell);
+            for (int d = 0; d < 3; d++) uc[d] = face_pushed(D, d, cell, pushed);
 #pragma unroll
             for (int j = 0; j < 6; j++) {
                 nty[j] = GAS_T, np[j] = 0.0f;
                 if (nbr[j] != NONE) nty[j] = cfv(D, F_TYPE, nbr[j]), np[j] = cfv(D, F_P, nbr[j]);
             }
 #pragma unroll
-            for (int d = 0; d < 3; d++) nu[d] = nbr[2 * d + 1] != NONE ? cfv(D, F_U + d, nbr[2 * d + 1]) : 0.0f;
+            for (int d = 0; d < 3; d++) nu[d] = nbr[2 * d + 1] != NONE ? face_pushed(D, d, nbr[2 * d + 1], pushed) : 0.0f;
             const bool water = ty == WATER_T;
             sts_f(dl + 4u * L.at[k], water ? 1.0f : 0.0f);  // for the masks below
             C.r[k] = 0.0f, C.p[k] = pc, C.d[k] = water ? dold : 0.0f, C.q[k] = 0.0f, C.z[k] = 0.0f, bq[k] = 0.0f;
@@ -677,16 +678,6 @@ __global__ void __launch_bounds__(SOLVE_T, 2) k_solve_batch(const Dev* __restric
     uint32_t n_recs;
     SolveRec* recs = solve_recs(n_recs);
     solve_body<FP64>(s_dev, blockIdx.x - s_c0[job], s_c0[job + 1] - s_c0[job], recs, n_recs);
-}
-
-// Every scene's grid barrier counter back to zero before the joint solve (a one-scene step
-// clears its own in k_bullet_apply), and its last solve's iterations set aside for the split: the
-// solve itself rewrites them, and every CTA must compute the same split.
-__global__ void k_solve_reset_m(Multi M) {
-    __shared__ Dev sD;
-    __shared__ Cta c;
-    multi_cta(M, sD, c);
-    if (threadIdx.x == 0) sD.st->bar_count = 0u, sD.st->iters_prev = sD.st->s.solve_iters;
 }
 
 }  // namespace ntr

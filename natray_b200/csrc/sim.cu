@@ -313,7 +313,6 @@ static ntr_status allocate(Sim& S) {
     D.outlines = ol;
     AL(D.sections, NTR_MAX_SHOTS * NTR_N_SEC);
     AL(D.bullet_hit, NTR_MAX_SHOTS * NTR_HIT_FIELDS);
-    AL(D.bullet_prep, NTR_MAX_SHOTS * 4);
     AL(D.bullet_patch, NTR_MAX_SHOTS * NTR_MAX_PATCHES * 4);
     AL(D.pose_log, NTR_MAX_SHOTS * NTR_LOG_CAP * 3);
     AL(D.spray, (size_t)D.spray_cap * 3);
@@ -369,6 +368,7 @@ static ntr_status upload_state(Sim& S, const World& w) {
     CU(cudaMemsetAsync(D.air[0], 0, (size_t)NTR_AIR_FIELDS * D.cap_cells * 4, S.stream));
     CU(cudaMemsetAsync(D.air[1], 0, (size_t)NTR_AIR_FIELDS * D.cap_cells * 4, S.stream));
     CU(cudaMemsetAsync(D.block_active, 0, (size_t)D.cap_blocks * 4, S.stream));
+    CU(cudaMemsetAsync(D.cta_sum, 0, ((size_t)D.scan_ctas + 1) * 8, S.stream));  // of no step
     const int cur = (int)(h.state.step & 1u);
     const uint32_t nbp = h.n_blocks_prev;
     {
@@ -600,10 +600,8 @@ static uint64_t enqueue_step(Sim& S, cudaStream_t s, uint32_t n_mem, uint32_t n_
     // The spray's flight reads only the spray, the step length and the spray count from before
     // this step's break-ups (k_spray_scan advances it): beside the sort too.
     LA(k_spray_update, G_cell, 256, D);
-    L(k_clear_mask, std::max((D.nwords + 255) / 256, 1u), 256, D);
     L(k_mark, (uint32_t)(((uint64_t)warp_round(D.Np) + warp_round(D.cap_blocks) + warp_round(D.Nv) + 255) / 256), 256, D);
-    L(k_scan_words_a, D.scan_ctas, SCAN_T, D);
-    L(k_scan_words_b, D.scan_ctas, SCAN_T, D);
+    L(k_scan_words, D.scan_ctas, SCAN_T, D);
     if (a != s) {
         cudaEventRecord(S.ev_fork[1], s);
         cudaStreamWaitEvent(a, S.ev_fork[1], 0);
@@ -636,14 +634,10 @@ static uint64_t enqueue_step(Sim& S, cudaStream_t s, uint32_t n_mem, uint32_t n_
     join(0);
     L(k_gather_prep, G_cell, 256, D);
     L(k_air_fill, G_cell, 256, D);
-    L(k_bullet_prep, n_shots, 32, D);
     {
         const dim3 gp((NTR_MAX_PATCHES + BULLET_PW - 1) / BULLET_PW, n_shots);
-        L(k_bullet_patch, gp, BULLET_PW * 32, D);
+        L(k_bullet, gp, BULLET_PW * 32, D);
     }
-    L(k_bullet_finish, n_shots, 256, D);
-    L(k_bullet_apply, G_cell, 256, D);
-    // (k_bullet_apply has set the pressure solve's grid barrier counter to zero.)
     n += enqueue_solve(S, s, nullptr, 1u, fp64, prof, grids.solve, grids.solve_dyn);
     L(k_project, G_cell, 256, D);
     L(k_extend_1, G_cell, 256, D);
