@@ -111,7 +111,8 @@ __device__ __forceinline__ void set_word_bits(uint32_t* mask, uint32_t word, uin
     if (bits && (__ffs(peers) - 1) == (int)(threadIdx.x & 31u)) atomicOr(mask + word, all);
 }
 // Sets the bits of `n` blocks in a row along z from `slot` (n <= 32; none where n is 0). Slots run
-// along z, so a row's bits are one word's, or for a row over a word's end two words'.
+// along z, so a row's bits are one word's, or for a row over a word's end two words'. (The row lies in
+// the domain, so the second word has bits only where it exists.)
 __device__ __forceinline__ void set_block_row(uint32_t* mask, uint32_t slot, uint32_t n) {
     const uint64_t bits = ((1ull << n) - 1ull) << (slot & 31u);
     set_word_bits(mask, slot >> 5, (uint32_t)bits);
@@ -137,6 +138,9 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
     auto clampb = [&](I3 b) {
         return I3{min(max(b.x, 0), bmax.x), min(max(b.y, 0), bmax.y), min(max(b.z, 0), bmax.z)};
     };
+    // A stencil end past the range of the cell numbers (a coordinate out of their range saturates)
+    // wraps, as in the reference's integers: hi then lies below lo, and there is no such row.
+    auto step_by = [](I3 c, uint32_t k) { return I3{(int32_t)((uint32_t)c.x + k), (int32_t)((uint32_t)c.y + k), (int32_t)((uint32_t)c.z + k)}; };
     const uint32_t np_w = warp_round(D.Np), nb_w = warp_round(D.cap_blocks);
     if (i < np_w) {
         // The up to 2x2x2 blocks of a particle's stencil.
@@ -147,8 +151,8 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
             float4 p = D.pos[i];
             alive = D.vel[i].w >= 0.5f;
             I3 c = own_cell(g, xyz(p));
-            lo = clampb(shr2(c - I3{1, 1, 1}));
-            hi = clampb(shr2(c + I3{2, 2, 2}));
+            lo = clampb(shr2(step_by(c, 0u - 1u)));
+            hi = clampb(shr2(step_by(c, 2u)));
             I3 ob = shr2(c);
             D.pslot[i] = (alive && in_bd(g, ob)) ? block_slot(g, ob) : NONE;
         }
@@ -157,7 +161,7 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const I3 b = {lo.x + (k & 1), lo.y + (k >> 1), lo.z};
-            const bool valid = alive && b.x <= hi.x && b.y <= hi.y;
+            const bool valid = alive && b.x <= hi.x && b.y <= hi.y && lo.z <= hi.z;
             set_block_row(mask, valid ? block_slot(g, b) : 0u, valid ? (uint32_t)(hi.z - lo.z + 1) : 0u);
         }
         return;
@@ -179,14 +183,14 @@ __device__ __forceinline__ void mark_body(const Dev& D, const CT& C) {
         dry = !(push.y <= 0.0f || on_water);
         if (dry) {
             I3 c = own_cell(g, xyz(D.mem_x[0][j]));
-            lo = clampb(shr2(c - I3{2, 2, 2}));
-            hi = clampb(shr2(c + I3{3, 3, 3}));
+            lo = clampb(shr2(step_by(c, 0u - 2u)));
+            hi = clampb(shr2(step_by(c, 3u)));
         }
     }
     if (!__any_sync(0xffffffffu, dry)) return;
     for (int k = 0; k < 9; k++) {
         const I3 b = {lo.x + k / 3, lo.y + k % 3, lo.z};
-        const bool valid = dry && b.x <= hi.x && b.y <= hi.y;
+        const bool valid = dry && b.x <= hi.x && b.y <= hi.y && lo.z <= hi.z;
         set_block_row(mask, valid ? block_slot(g, b) : 0u, valid ? (uint32_t)(hi.z - lo.z + 1) : 0u);
     }
 }

@@ -4,6 +4,7 @@ bullets waiting, flying and gone in one launch, and scenes with different number
 batch. All bit for bit."""
 import subprocess
 
+import numpy as np
 import pytest
 
 from natray_b200 import Params, World, build_world
@@ -48,6 +49,32 @@ def test_bullets_equal_the_oracle(preset):
     o, s = Oracle(w.blob), Sim(world=w)
     for _ in range(12):  # the first arrival and the others still waiting (0.5 ms apart)
         assert o.step(8) == s.step(8) == 8
+    same(World(o.snapshot()), s.snapshot())
+    s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("z", [1e30, -1e30, float("inf"), float("-inf")])
+@pytest.mark.parametrize("what", ["particle", "vertex"])
+def test_a_coordinate_past_the_cell_numbers_marks_no_block(what, z):
+    # A live particle, or a dry vertex (its triangles gone, so that nothing else feels it), at the
+    # domain's far corner in x and y and out of the range of 32-bit cell numbers in z: the row of
+    # blocks along z is inverted. (A row taken as its length would mark the blocks after it, and past
+    # the bitmask's end.)
+    w = World(world(Params(resolution=20, mesh_level=3, block_cap=4096, spray_cap=50000)).blob)
+    u = w.h.params
+    x, y = (u.origin[k] + (u.dims[k] - 0.5) * u.origin[3] for k in (0, 1))
+    if what == "particle":
+        w.sec("PARTICLES")[7, :3] = (x, y, z)
+        assert w.sec("PARTICLES")[7, 7] >= 0.5
+    else:
+        j = int(np.flatnonzero(w.sec("MEM_PUSH").reshape(-1, 2)[:, 1] > 0)[5])
+        w.sec("MEM_X")[j, :3] = (x, y, z)
+        w.sec("MEM_WATER")[j, 3] = 0.0
+        off = w.sec("VTRI_OFF")
+        w.sec("ALIVE")[w.sec("VTRI")[off[j] : off[j + 1]]] = 0
+    o, s = Oracle(w.blob), Sim(world=w)
+    assert o.step(2) == s.step(2) == 2
     same(World(o.snapshot()), s.snapshot())
     s.close()
 
