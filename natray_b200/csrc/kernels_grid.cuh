@@ -858,9 +858,16 @@ __device__ __forceinline__ void gather_prep_body(const Dev& D, const CT& C) {
         grid_prep_cell(D, g, knot, kr, dt, grav, cell, s8);
     }
     // The last step's block bitmask, which the air's carry was the last to read, is the next step's:
-    // its blocks' words are cleared here (a launch over the whole domain's bitmask before).
+    // its blocks' words are cleared here (a launch over the whole domain's bitmask before). Blocks past
+    // the capacity have bits but no place in the list: a step that filled the list may have left some,
+    // and its bitmask is cleared whole.
     const int old = cur_of(st) ^ 1;
-    for (uint32_t b = C.x() * blockDim.x + threadIdx.x; b < st->s.n_blocks_prev; b += C.nx() * blockDim.x) D.mask[old][D.block_list[old][b] >> 5] = 0u;
+    const uint32_t n_prev = st->s.n_blocks_prev, t0 = C.x() * blockDim.x + threadIdx.x, nt = C.nx() * blockDim.x;
+    if (n_prev < min(D.cap_blocks, U->bdims[3])) {
+        for (uint32_t b = t0; b < n_prev; b += nt) D.mask[old][D.block_list[old][b] >> 5] = 0u;
+    } else {
+        for (uint32_t w = t0; w < D.nwords; w += nt) D.mask[old][w] = 0u;
+    }
 }
 __global__ void k_gather_prep(Dev D) { gather_prep_body(D, HwCta{}); }
 __global__ void k_gather_prep_m(Multi M) {

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from natray_b200 import Params, World, build_world
+from natray_b200._abi import NatrayError
 from natray_b200.batch import Batch
 from natray_b200.sim import Sim
 from oracle.py import Oracle
@@ -75,6 +76,26 @@ def test_a_coordinate_past_the_cell_numbers_marks_no_block(what, z):
         w.sec("ALIVE")[w.sec("VTRI")[off[j] : off[j + 1]]] = 0
     o, s = Oracle(w.blob), Sim(world=w)
     assert o.step(2) == s.step(2) == 2
+    same(World(o.snapshot()), s.snapshot())
+    s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cut", [1, 4, 8])
+def test_steps_past_an_overflow_equal_the_oracle(cut):
+    # A low balloon falling, with fewer blocks of capacity than it takes: the steps go on with the blocks
+    # that fit (the call reports the overflow), and a block past the capacity in one step is no block of
+    # the steps after unless they mark it too. One call on either side: nothing adapts in between.
+    p = dict(resolution=16, mesh_level=3, spray_cap=100000, height=0.12)
+    o = Oracle(world(Params(block_cap=4096, **p)).blob)
+    o.step(1)
+    w = world(Params(block_cap=World(o.snapshot()).state["n_blocks"] - cut, **p))
+    o, s = Oracle(w.blob), Sim(world=w)
+    with pytest.raises(RuntimeError):
+        o.step(120)
+    with pytest.raises(NatrayError) as e:
+        s.step(120)
+    assert e.value.status == 3  # NTR_E_OVERFLOW
     same(World(o.snapshot()), s.snapshot())
     s.close()
 
