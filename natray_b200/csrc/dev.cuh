@@ -88,7 +88,7 @@ struct DevState {
     uint32_t solver_on;
     uint32_t ticket[4];  // per bullet: its CTAs that are done (k_bullet)
     uint32_t nbrk;       // break-ups of this step
-    uint32_t err;        // bit 0: a bounded grid barrier gave up
+    uint32_t err;        // bit 0: a bounded wait gave up (the solve's barrier, the scan's); no step is taken until a restore
     uint32_t bar_count;  // grid barrier of the persistent solver: arrivals (reset per launch)
     uint32_t iters_prev;  // the last solve's iterations, kept for a joint solve's split
     // The next block P2G (0) and G2P (1) hand out in a one-scene launch, zeroed by k_begin_step.
@@ -114,9 +114,10 @@ struct Dev {
     float4 *pos, *vel, *c0, *c1, *c2;
     uint32_t Np, Nv, Nt, cap_blocks, cap_cells, nwords, spray_cap, wet_res;
     uint32_t n_tiles, radix_passes, scan_ctas, fp64_dots;
-    // The solver's grid barriers: polls before a wait gives up, and a CTA that skips its first
-    // arrival (NONE: none) so that the others' waits run out (ntr_sim_test_barrier).
-    uint32_t bar_spins, bar_skip;
+    // The waits for other CTAs (the solver's grid barriers, the bitmask's scan): polls before one
+    // gives up, a CTA of the solve that skips its first arrival and a CTA of the scan that keeps its
+    // count (NONE: none) so that the others' waits run out (ntr_sim_test_barrier, ntr_sim_test_scan).
+    uint32_t bar_spins, bar_skip, scan_skip;
     uint32_t* mask[2];
     uint32_t* prefix[2];
     uint32_t* block_list[2];

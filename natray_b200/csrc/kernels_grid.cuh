@@ -25,6 +25,10 @@ __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
         s.dt_ns = 0;
         return;
     }
+    if (D.st->err != 0u) {  // a wait of an earlier step gave up: no step on what it left
+        s.dt_ns = 0;
+        return;
+    }
     float vmax = s.max_speed;
     uint32_t arrive = U->limits[3];
     for (uint32_t k = 0; k < U->mem[3]; k++) {
@@ -210,16 +214,22 @@ constexpr int SCAN_T = 256, SCAN_W = 8;  // 2048 words per CTA
 // counts of those before it as they come (each with the number of its step beside it, in a word
 // written whole; a CTA waits only for CTAs that were launched before it, at most D.bar_spins polls).
 // Two launches before, the counts and then the rest: the second one waited 4 us for the first.
+// A CTA whose wait gives up (or sees that another's has) numbers nothing: it sets the error bit, takes
+// the blocks' count back and ends the step, whose other kernels all do nothing at a step length of zero.
 template <class CT>
 __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
     DevState* st = D.st;
-    if (st->s.dt_ns == 0) return;
+    // One thread's reading of the step length for the whole CTA: another CTA may zero it meanwhile.
+    __shared__ uint32_t s_live;
+    if (threadIdx.x == 0) s_live = *(volatile uint32_t*)&st->s.dt_ns;
+    __syncthreads();
+    if (s_live == 0u) return;
     const int cur = cur_of(st);
     const uint32_t* m = D.mask[cur];
     uint32_t* prefix = D.prefix[cur];
     uint32_t* list = D.block_list[cur];
     const unsigned long long tag = ((unsigned long long)st->s.step << 1) | 1ull;  // above 31 bits of count; a new state's words, zero, match none
-    __shared__ uint32_t s_base, ws[SCAN_T / 32];
+    __shared__ uint32_t s_base, s_ok, ws[SCAN_T / 32];
     // Each thread owns SCAN_W consecutive words (two 16-byte loads where all are in range).
     static_assert(SCAN_W == 8, "two uint4 per thread");
     uint32_t w0 = C.x() * SCAN_T * SCAN_W + threadIdx.x * SCAN_W;
@@ -245,22 +255,33 @@ __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
         if (lane == 0) {
             uint32_t t = 0;
             for (int k = 0; k < SCAN_T / 32; k++) t += ws[k];
-            *(volatile unsigned long long*)(D.cta_sum + C.x()) = (tag << 31) | t;
+            if (C.x() != D.scan_skip) *(volatile unsigned long long*)(D.cta_sum + C.x()) = (tag << 31) | t;
         }
         uint32_t t = 0;
-        for (uint32_t k = lane; k < C.x(); k += 32) {
+        bool ok = true;
+        for (uint32_t k = lane; ok && k < C.x(); k += 32) {
             unsigned long long v;
             for (uint32_t spins = 0; ((v = *(volatile const unsigned long long*)(D.cta_sum + k)) >> 31) != tag;)
-                if (++spins > D.bar_spins) {
-                    atomicOr(&st->err, 1u);
+                if (++spins > D.bar_spins || ((spins & 1023u) == 0u && *(volatile uint32_t*)&st->err != 0u)) {
+                    ok = false;
                     break;
                 }
             t += (uint32_t)v & 0x7fffffffu;
         }
+        ok = __all_sync(0xffffffffu, ok);
         for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        if (lane == 0) s_base = t;
+        if (lane == 0) s_base = t, s_ok = ok;
     }
     __syncthreads();
+    if (!s_ok) {
+        if (threadIdx.x == 0) {
+            atomicOr(&st->err, 1u);
+            __threadfence();  // the error before the count: the last CTA writes the count, then looks for the error
+            *(volatile uint32_t*)&st->s.n_blocks = 0u;
+            *(volatile uint32_t*)&st->s.dt_ns = 0u;
+        }
+        return;
+    }
     uint32_t wbase = 0;
     for (uint32_t k = 0; k < warp; k++) wbase += ws[k];
     uint32_t run = s_base + wbase + inc - cnt;
@@ -280,8 +301,10 @@ __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
         }
     }
     if (C.x() == C.nx() - 1 && threadIdx.x == SCAN_T - 1) {
-        st->s.n_blocks = run;
+        *(volatile uint32_t*)&st->s.n_blocks = run;
         if (run > cap) st->s.overflow = 1u;
+        __threadfence();
+        if (*(volatile uint32_t*)&st->err != 0u) *(volatile uint32_t*)&st->s.n_blocks = 0u;
     }
 }
 __global__ void __launch_bounds__(SCAN_T) k_scan_words(Dev D) { scan_words_body(D, HwCta{}); }

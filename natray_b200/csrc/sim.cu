@@ -252,7 +252,7 @@ static ntr_status allocate(Sim& S) {
     D.radix_passes = radix_passes_for(D.cap_blocks);
     D.fp64_dots = S.fp64;
     D.bar_spins = BARRIER_SPINS;
-    D.bar_skip = NONE;
+    D.bar_skip = D.scan_skip = NONE;
     ntr_status r;
 #define AL(p, n) \
     if ((r = S.alloc(p, n)) != NTR_OK) return r
@@ -1248,11 +1248,12 @@ NTR_API ntr_status ntr_sim_autotune(ntr_sim* sim, uint32_t steps, ntr_tuning* be
     return NTR_OK;
 }
 
-NTR_API ntr_status ntr_sim_test_barrier(ntr_sim* sim, uint32_t spins, uint32_t skip_cta) {
+static ntr_status test_waits(ntr_sim* sim, uint32_t spins, uint32_t bar_skip, uint32_t scan_skip) {
     GUARD(sim);
     CU(cudaStreamSynchronize(S.stream));
     S.D.bar_spins = spins ? spins : BARRIER_SPINS;
-    S.D.bar_skip = skip_cta;
+    S.D.bar_skip = bar_skip;
+    S.D.scan_skip = scan_skip;
     // The kernels take the pointer table by value: the captured step graphs hold the old one.
     for (auto& kv : S.graphs) {
         if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -1261,6 +1262,8 @@ NTR_API ntr_status ntr_sim_test_barrier(ntr_sim* sim, uint32_t spins, uint32_t s
     S.graphs.clear();
     return NTR_OK;
 }
+NTR_API ntr_status ntr_sim_test_barrier(ntr_sim* sim, uint32_t spins, uint32_t skip_cta) { return test_waits(sim, spins, skip_cta, NONE); }
+NTR_API ntr_status ntr_sim_test_scan(ntr_sim* sim, uint32_t spins, uint32_t skip_cta) { return test_waits(sim, spins, NONE, skip_cta); }
 
 NTR_API ntr_status ntr_sim_work(ntr_sim* sim, uint64_t out[NTR_WORK_FIELDS], int reset) {
     GUARD(sim);
