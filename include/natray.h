@@ -425,7 +425,7 @@ NTR_API ntr_status ntr_sim_work(ntr_sim* s, uint64_t out[NTR_WORK_FIELDS], int r
  * context stays usable, and the state is that of a failed step (restore a snapshot). */
 NTR_API ntr_status ntr_sim_test_barrier(ntr_sim* s, uint32_t spins, uint32_t skip_cta);
 /* The same for the scan of the block bitmask, whose CTAs wait for the counts of those before them:
- * CTA `skip_cta` of the scan keeps its count to itself. The step in which a wait gives up ends
+ * the CTA at place `skip_cta` of the scan keeps its count to itself. The step in which a wait gives up ends
  * there, with no blocks; the later steps of the call, and of calls before a restore, are not taken. */
 NTR_API ntr_status ntr_sim_test_scan(ntr_sim* s, uint32_t spins, uint32_t skip_cta);
 /* Kernel launches made by the last ntr_sim_step call, and its device time in ms. */

@@ -115,13 +115,13 @@ struct Dev {
     uint32_t Np, Nv, Nt, cap_blocks, cap_cells, nwords, spray_cap, wet_res;
     uint32_t n_tiles, radix_passes, scan_ctas, fp64_dots;
     // The waits for other CTAs (the solver's grid barriers, the bitmask's scan): polls before one
-    // gives up, a CTA of the solve that skips its first arrival and a CTA of the scan that keeps its
+    // gives up, a CTA of the solve that skips its first arrival and a place of the scan that keeps its
     // count (NONE: none) so that the others' waits run out (ntr_sim_test_barrier, ntr_sim_test_scan).
     uint32_t bar_spins, bar_skip, scan_skip;
     uint32_t* mask[2];
     uint32_t* prefix[2];
     uint32_t* block_list[2];
-    unsigned long long* cta_sum;  // per CTA of the bitmask's scan: the step, and below it its words' bits
+    unsigned long long* cta_sum;  // per place of the bitmask's scan: the step, and below it its words' bits; last, the next place
     uint32_t *pslot, *key, *key_alt, *val_alt, *key_sorted, *sorted, *hist;
     uint32_t* hist2;  // the sort's second histogram (pass 1's, counted by pass 0's scatter)
     uint32_t *block_start, *block_nb, *block_active;

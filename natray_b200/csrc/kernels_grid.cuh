@@ -17,6 +17,7 @@ __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
     D.st->next_block[0] = D.st->next_block[1] = 0u;
     D.st->pushed = 0u;
     D.st->bar_count = 0u;  // the pressure solve's grid barrier
+    D.cta_sum[D.scan_ctas] = 0ull;  // the bitmask scan's places
     D.st->iters_prev = D.st->s.solve_iters;  // for a joint solve's split: every CTA must compute the same one
     const ntr_gpu_params* U = D.U;
     ntr_state& s = D.st->s;
@@ -212,7 +213,8 @@ constexpr int SCAN_T = 256, SCAN_W = 8;  // 2048 words per CTA
 
 // One launch: a CTA counts its words' bits, leaves the count for the CTAs after it and takes the
 // counts of those before it as they come (each with the number of its step beside it, in a word
-// written whole; a CTA waits only for CTAs that were launched before it, at most D.bar_spins polls).
+// written whole). A CTA takes its place when it starts, from a counter, not from its index: so it waits
+// only for CTAs that run or are done, in whatever order they start, at most D.bar_spins polls.
 // Two launches before, the counts and then the rest: the second one waited 4 us for the first.
 // A CTA whose wait gives up (or sees that another's has) numbers nothing: it sets the error bit, takes
 // the blocks' count back and ends the step, whose other kernels all do nothing at a step length of zero.
@@ -220,10 +222,14 @@ template <class CT>
 __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
     DevState* st = D.st;
     // One thread's reading of the step length for the whole CTA: another CTA may zero it meanwhile.
-    __shared__ uint32_t s_live;
-    if (threadIdx.x == 0) s_live = *(volatile uint32_t*)&st->s.dt_ns;
+    __shared__ uint32_t s_live, s_place;
+    if (threadIdx.x == 0) {
+        s_live = *(volatile uint32_t*)&st->s.dt_ns;
+        s_place = (uint32_t)atomicAdd(&D.cta_sum[D.scan_ctas], 1ull);
+    }
     __syncthreads();
     if (s_live == 0u) return;
+    const uint32_t place = s_place;
     const int cur = cur_of(st);
     const uint32_t* m = D.mask[cur];
     uint32_t* prefix = D.prefix[cur];
@@ -232,7 +238,7 @@ __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
     __shared__ uint32_t s_base, s_ok, ws[SCAN_T / 32];
     // Each thread owns SCAN_W consecutive words (two 16-byte loads where all are in range).
     static_assert(SCAN_W == 8, "two uint4 per thread");
-    uint32_t w0 = C.x() * SCAN_T * SCAN_W + threadIdx.x * SCAN_W;
+    uint32_t w0 = place * SCAN_T * SCAN_W + threadIdx.x * SCAN_W;
     uint32_t words[SCAN_W], cnt = 0;
     if (w0 + SCAN_W <= D.nwords) {
         const uint4 a = *reinterpret_cast<const uint4*>(m + w0), b = *reinterpret_cast<const uint4*>(m + w0 + 4);
@@ -255,11 +261,11 @@ __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
         if (lane == 0) {
             uint32_t t = 0;
             for (int k = 0; k < SCAN_T / 32; k++) t += ws[k];
-            if (C.x() != D.scan_skip) *(volatile unsigned long long*)(D.cta_sum + C.x()) = (tag << 31) | t;
+            if (place != D.scan_skip) *(volatile unsigned long long*)(D.cta_sum + place) = (tag << 31) | t;
         }
         uint32_t t = 0;
         bool ok = true;
-        for (uint32_t k = lane; ok && k < C.x(); k += 32) {
+        for (uint32_t k = lane; ok && k < place; k += 32) {
             unsigned long long v;
             for (uint32_t spins = 0; ((v = *(volatile const unsigned long long*)(D.cta_sum + k)) >> 31) != tag;)
                 if (++spins > D.bar_spins || ((spins & 1023u) == 0u && *(volatile uint32_t*)&st->err != 0u)) {
@@ -300,7 +306,7 @@ __device__ __forceinline__ void scan_words_body(const Dev& D, const CT& C) {
             run++;
         }
     }
-    if (C.x() == C.nx() - 1 && threadIdx.x == SCAN_T - 1) {
+    if (place == C.nx() - 1 && threadIdx.x == SCAN_T - 1) {
         *(volatile uint32_t*)&st->s.n_blocks = run;
         if (run > cap) st->s.overflow = 1u;
         __threadfence();
