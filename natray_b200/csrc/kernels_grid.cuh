@@ -14,6 +14,7 @@ namespace ntr {
 template <class CT>
 __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
     if (threadIdx.x != 0 || C.x() != 0) return;
+    const uint32_t budget = D.st->step_budget, err = D.st->err;  // loaded together: one trip to memory
     D.st->next_block[0] = D.st->next_block[1] = 0u;
     D.st->pushed = 0u;
     D.st->bar_count = 0u;  // the pressure solve's grid barrier
@@ -21,12 +22,12 @@ __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
     D.st->iters_prev = D.st->s.solve_iters;  // for a joint solve's split: every CTA must compute the same one
     const ntr_gpu_params* U = D.U;
     ntr_state& s = D.st->s;
-    if (D.st->step_budget == 0u) {  // a batch scene that has taken its steps of the call
+    if (budget == 0u) {  // a batch scene that has taken its steps of the call
         if (!D.st->parked) D.st->parked = 1u, D.st->parked_dt = s.dt_ns;
         s.dt_ns = 0;
         return;
     }
-    if (D.st->err != 0u) {  // a wait of an earlier step gave up: no step on what it left
+    if (err != 0u) {  // a wait of an earlier step gave up: no step on what it left
         s.dt_ns = 0;
         return;
     }
@@ -53,7 +54,6 @@ __device__ __forceinline__ void begin_step_body(const Dev& D, const CT& C) {
     if (s.free_dt_ns > 0u) dt_s = mn(dt_s, 1.25f * (float)s.free_dt_ns * 1e-9f);
     uint32_t free_ns = max(f2u(dt_s * 1e9f), 20u);
     uint32_t stop = U->limits[3];
-    const uint32_t budget = D.st->step_budget;
     bool live = s.t_ns < stop;
     uint32_t dt_ns = 0;
     if (live) {
