@@ -154,13 +154,15 @@ def algorithmic_bytes(kernel: str, st: dict, n_particles: int, iters: int) -> fl
     """Bytes a launch of `kernel` must move at the least, from the per-unit figures of the step:
     P2G reads a particle's 80 B and its index and writes its cells' particle counts (its tile of
     sums is this implementation's, not the algorithm's: the cells' sums are written by the tile
-    gather); the solve reads d, z, diag, type, p, r, q and writes d', q, p, r, z per water cell
-    and iteration (48 B) and sets up with 40 B per water cell; G2P reads a particle's 80 B, its
+    gather); the solve keeps its values on the chip: per water cell it reads the type, pressure,
+    source, three velocities and old direction once and leaves the diagonal, p, r, q and z (48 B),
+    and per iteration it writes the cell's residual and reads its share of the 96 across its block's
+    faces (10 B); G2P reads a particle's 80 B, its
     index and its cells' 8 fields once (32 B per cell) and writes the particle's 80 B."""
     cells = st["n_blocks"] * 64
     if kernel.startswith("k_solve"):
         n_water = st.get("_n_water", cells)
-        return 48.0 * n_water * max(iters, 1) + 40.0 * n_water
+        return 10.0 * n_water * max(iters, 1) + 48.0 * n_water
     if kernel == "k_p2g":
         return 84.0 * n_particles + 4.0 * cells
     if kernel.startswith("k_g2p"):
@@ -358,7 +360,7 @@ def run_native(args, rank, world, local):
             "step_roofline": {"bound": "hbm", "achieved": step_bytes / t_dev / 1e9 * world, "peak": peak, "unit": "GB/s",
                               "frac": step_bytes / t_dev / 1e9 / peak, "peak_kind": peak_kind,
                               "algorithmic_bytes_per_step": step_bytes / max(work["steps"], 1), "work": work,
-                              "note": "sum over the timed steps of 160 Np + 160 cells + 48 K Nw + (256 Nv + 32 Nt) Sm "
+                              "note": "sum over the timed steps of 160 Np + 160 cells + 10 K Nw + (256 Nv + 32 Nt) Sm "
                                       "+ 44 Sa Na + 48 Nspray, counted on the device by the steps, over their device time"},
             "kernel_shares": shares,
             "clocks": clk.summary(),

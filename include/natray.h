@@ -411,7 +411,7 @@ NTR_API ntr_status ntr_sim_profile(ntr_sim* s, uint32_t n, uint32_t stop_ns, cha
  * taken; cells of their blocks (64 per block, summed over the steps); water cells times solver
  * iterations; rubber substeps; free-gas cells times air substeps; spray slots in use. The
  * algorithmic bytes of those steps follow from them (160 per particle and step, 160 per cell,
- * 48 per water cell and iteration, 256 per vertex and 32 per triangle and rubber substep, 44 per
+ * 10 per water cell and iteration, 256 per vertex and 32 per triangle and rubber substep, 44 per
  * gas cell and air substep, 48 per spray slot): the per-step quantities the reference's
  * profiler sees through its State readback (src/sim.rs:594-689). Waits for the stream. */
 #define NTR_WORK_FIELDS 6

@@ -186,10 +186,12 @@ class Sim:
     def algorithmic_bytes(self, work: dict) -> float:
         """Bytes the steps counted in `work` must move at the least: 160 per particle and step
         (its state read and written), 160 per block cell (transfer sums, cell fields, projection,
-        the G2P read, the clear), 48 per water cell and solver iteration, 256 per vertex and 32
-        per triangle and rubber substep, 44 per gas cell and air substep, 48 per spray slot."""
+        the G2P read, the clear), 10 per water cell and solver iteration (its residual out, and the
+        96 residuals across a block's faces in: 4 + 96 * 4 / 64; the rest stays on the chip), 256
+        per vertex and 32 per triangle and rubber substep, 44 per gas cell and air substep, 48 per
+        spray slot."""
         i = self.info
-        return (160.0 * i.n_particles * work["steps"] + 160.0 * work["cells"] + 48.0 * work["water_iters"]
+        return (160.0 * i.n_particles * work["steps"] + 160.0 * work["cells"] + 10.0 * work["water_iters"]
                 + (256.0 * i.n_verts + 32.0 * i.n_tris) * work["mem_substeps"] + 44.0 * work["gas_substeps"]
                 + 48.0 * work["spray"])
 
