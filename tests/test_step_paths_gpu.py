@@ -1,8 +1,10 @@
 """The step's paths that depend on sizes: the pressure solve with one block a warp (registers),
 several (records in shared memory) and more than the shared memory holds (records in global memory);
 bullets waiting, flying and gone in one launch, and scenes with different numbers of them in one
-batch. All bit for bit."""
+batch; coordinates and block counts past their range; the quotients. All bit for bit."""
+import ctypes as C
 import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -10,6 +12,7 @@ import pytest
 from natray_b200 import Params, World, build_world
 from natray_b200._abi import NatrayError
 from natray_b200.batch import Batch
+from natray_b200.build import ARCH, NVCC
 from natray_b200.sim import Sim
 from oracle.py import Oracle
 
@@ -116,37 +119,82 @@ def test_batch_of_scenes_with_different_numbers_of_bullets():
         s.close()
 
 
-def test_quotient_by_the_reciprocal_is_the_quotient(tmp_path):
-    # div_by of dev.cuh restated: a / b for |a| in [2^-80, 2^40], b in [2^-60, 2^40], ends of the
-    # mantissas included.
-    src = tmp_path / "d.cpp"
-    src.write_text(r"""
-#include <cmath>
-#include <cstdint>
-#include <cstdio>
-#include <cstring>
-int main() {
-    uint64_t s = 88172645463325252ull; long bad = 0;
-    for (long t = 0; t < 20000000; t++) {
-        s ^= s << 13, s ^= s >> 7, s ^= s << 17;
-        uint32_t ma = s & 0x7fffff, mb = (s >> 23) & 0x7fffff;
-        const int ea = (int)((s >> 46) % 121) - 80, eb = (int)((s >> 54) % 101) - 60;
-        if ((t & 7) == 0) mb = 0x7fffff;
-        if ((t & 7) == 1) mb = (s >> 40) & 0xff;
-        if ((t & 7) == 2) ma = 0x7fffff - ((s >> 50) & 3);
-        float a = std::ldexp(1.0f + ma * 0x1p-23f, ea);
-        const float b = std::ldexp(1.0f + mb * 0x1p-23f, eb);
-        if (s >> 63) a = -a;
-        const float y = 1.0f / b, want = a / b;
-        float q = a * y;
-        float e = std::fma(-q, b, a);
-        q = std::fma(e, y, q);
-        e = std::fma(-q, b, a);
-        q = std::fma(e, y, q);
-        bad += std::memcmp(&q, &want, 4) != 0;
-    }
-    std::printf("%ld\n", bad);
+# div_by (quotient.cuh) over pairs (a, b), with y = 1 / b as its callers keep it, against a / b.
+QUOTIENTS = r"""
+#ifdef __CUDACC__
+#include "quotient.cuh"
+__global__ void quotients(const float* a, const float* b, float* q, float* want, long n) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        q[i] = ntr::div_by(a[i], b[i], 1.0f / b[i]), want[i] = a[i] / b[i];
 }
-""")
-    subprocess.run(["g++", "-O2", "-march=native", "-ffp-contract=off", str(src), "-o", str(tmp_path / "d")], check=True)
-    assert subprocess.run([str(tmp_path / "d")], capture_output=True, text=True, check=True).stdout.strip() == "0"
+extern "C" int run(const float* a, const float* b, float* q, float* want, long n) {
+    quotients<<<1184, 256>>>(a, b, q, want, n);
+    return (int)cudaDeviceSynchronize();
+}
+#else
+#include <cmath>
+#define __device__
+#define __noinline__ __attribute__((noinline))
+#define __forceinline__ inline
+static inline float __fmaf_rn(float a, float b, float c) { return std::fmaf(a, b, c); }
+#include "quotient.cuh"
+extern "C" int run(const float* a, const float* b, float* q, float* want, long n) {
+    for (long i = 0; i < n; i++) q[i] = ntr::div_by(a[i], b[i], 1.0f / b[i]), want[i] = a[i] / b[i];
+    return 0;
+}
+#endif
+"""
+
+
+def quotient_pairs() -> tuple[np.ndarray, np.ndarray]:
+    """Numerators and denominators: every pair of the ends of div_by's range (2^-80, 2^-60, 2^40) with a
+    few ulp to either side, zeros of both signs, subnormals, the largest and infinite, NaN; and random
+    ones around the range and of any size, mantissas at their ends among them."""
+    ends = [np.float32(2.0) ** e for e in (-149, -126, -80, -60, 0, 40, 127)]
+    special = [0.0, 1e-40, 3.0, 7.0, 1.0 / 3.0, np.finfo(np.float32).max, np.inf, np.nan]
+    near = [np.uint32(np.float32(e).view(np.uint32) + d).view(np.float32) for e in ends for d in (0, 1, 2)]
+    near += [np.uint32(np.float32(e).view(np.uint32) - d).view(np.float32) for e in ends[1:] for d in (1, 2)]
+    v = np.array(special + near, dtype=np.float32)
+    v = np.concatenate([v, -v])
+    a, b = (x.ravel() for x in np.meshgrid(v, v))
+    r = np.random.default_rng(5)
+    n = 1 << 22
+
+    def some(lo: int, hi: int) -> np.ndarray:
+        m = r.integers(0, 1 << 23, n, dtype=np.uint32)
+        m[::8] = 0x7FFFFF
+        m[1::8] = r.integers(0, 256, m[1::8].size)
+        m[2::8] = 0x7FFFFF - r.integers(0, 4, m[2::8].size)
+        return r.permutation((m | (r.integers(lo + 127, hi + 127, n, dtype=np.uint32) << np.uint32(23))).view(np.float32))
+
+    sign = np.where(r.random(2 * n) < 0.5, np.float32(-1), np.float32(1))
+    return (np.concatenate([a, np.concatenate([some(-84, 44), some(-126, 128)]) * sign]).astype(np.float32),
+            np.concatenate([b, some(-63, 43), some(-126, 128)]).astype(np.float32))
+
+
+@pytest.mark.parametrize("where", ["host", pytest.param("device", marks=pytest.mark.gpu)])
+def test_quotient_by_the_reciprocal_is_the_quotient(tmp_path, where):
+    # The step's own source, compiled for the host (IEEE division and fused multiply-add there) and for
+    # the device: the same bits as a / b, NaN for NaN.
+    csrc = Path(__file__).resolve().parent.parent / "natray_b200" / "csrc"
+    src, so = tmp_path / ("q.cu" if where == "device" else "q.cpp"), tmp_path / "q.so"
+    src.write_text(QUOTIENTS)
+    if where == "device":
+        cmd = [NVCC, *ARCH, "-O3", "-fmad=false", "-shared", "-Xcompiler", "-fPIC"]
+    else:
+        cmd = ["g++", "-O2", "-march=native", "-ffp-contract=off", "-shared", "-fPIC"]
+    subprocess.run([*cmd, "-I", str(csrc), str(src), "-o", str(so)], check=True)
+    a, b = quotient_pairs()
+    if where == "device":
+        import torch
+        t = [torch.from_numpy(x).cuda() for x in (a, b)] + [torch.empty(a.size, dtype=torch.float32, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+        assert C.CDLL(str(so)).run(*(C.c_void_p(x.data_ptr()) for x in t), C.c_long(a.size)) == 0
+        q, want = t[2].cpu().numpy(), t[3].cpu().numpy()
+        with np.errstate(all="ignore"):
+            assert np.array_equal(want, a / b, equal_nan=True)  # the device's division itself
+    else:
+        q, want = np.empty_like(a), np.empty_like(a)
+        assert C.CDLL(str(so)).run(*(C.c_void_p(x.ctypes.data) for x in (a, b, q, want)), C.c_long(a.size)) == 0
+    bad = np.flatnonzero((q.view(np.uint32) != want.view(np.uint32)) & ~(np.isnan(q) & np.isnan(want)))
+    assert bad.size == 0, [(a[i], b[i], q[i], want[i]) for i in bad[:4]]
