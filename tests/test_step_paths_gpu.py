@@ -3,6 +3,7 @@ several (records in shared memory) and more than the shared memory holds (record
 bullets waiting, flying and gone in one launch, and scenes with different numbers of them in one
 batch; coordinates and block counts past their range; the quotients. All bit for bit."""
 import ctypes as C
+import re
 import subprocess
 from pathlib import Path
 
@@ -29,19 +30,31 @@ def world(p: Params) -> World:
     return World(Oracle(build_world(p).blob).snapshot())  # the measuring substep taken once, on the CPU
 
 
+def solve_storage(n_blocks: int, ctas: int) -> set:
+    """Where the CTAs of a solve of `n_blocks` keep their blocks: CTA c owns those of residues c, c + ctas,
+    ... (mod 256); registers while each warp has at most one, then the records its shared memory holds."""
+    src = (Path(__file__).resolve().parent.parent / "natray_b200" / "csrc" / "kernels_solve.cuh").read_text()
+    warps = int(re.search(r"constexpr int SOLVE_W = (\d+);", src).group(1))
+    records = int(re.search(r"SOLVE_DYN = (\d+)u \* sizeof\(SolveRec\);", src).group(1))
+    mine = np.bincount(np.arange(n_blocks) % 256 % ctas, minlength=ctas)
+    return {"registers" if m <= warps else "shared" if m <= records else "global" for m in mine}
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("fp64", [True, False])
-@pytest.mark.parametrize("ctas", [1, 2, 7, 40])
-def test_solve_with_blocks_in_registers_shared_and_global_memory(ctas, fp64):
+@pytest.mark.parametrize("ctas,where", [(1, {"global"}), (2, {"global"}), (4, {"global"}), (5, {"shared"}), (7, {"shared"}), (16, {"registers", "shared"}),
+                                        (40, {"registers"})])
+def test_solve_with_blocks_in_registers_shared_and_global_memory(ctas, where, fp64):
     w = world(Params(resolution=40, mesh_level=3, block_cap=4096, spray_cap=50000, dt_max=2e-6))
     out = []
     for n in (0, ctas):
         s = Sim(world=w, fp64_reductions=fp64)
         if n:
             s.tuning = {"solve_ctas": n, "cell_ctas_per_sm": 0, "block_ctas_per_sm": 0}
-        assert s.step(3) == 3 and s.step(3) == 3
+        for _ in range(2):
+            assert s.step(3) == 3
+            assert solve_storage(s.state["n_blocks"], n or 43) == (where if n else {"registers"})  # by default 43: 512 blocks, 12 a CTA
         out.append(s.snapshot())
-        assert s.state["n_blocks"] > 12 * 7  # 1 and 2 CTAs: more blocks than records in shared memory
         s.close()
     same(*out)
 
