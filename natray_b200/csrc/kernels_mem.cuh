@@ -1038,7 +1038,8 @@ __global__ void k_mem_tri_m(Multi M, uint32_t i, int par) {
     mem_tri_body(sD, c, par);
 }
 // Two CTAs an SM (128 registers): at the 255 that the contact search would take, one, the 64 scenes'
-// substeps took 838 us a step instead of 604.
+// substeps took 838 us a step, so bounded 610 (604 before the search kept its best sample's response;
+// with the bullets in the rubber of some of the scenes 747 against 762 before). The search spills for it.
 __global__ void __launch_bounds__(256, 2) k_mem_substep_m(Multi M, uint32_t k, int par) {
     __shared__ Dev sD;
     __shared__ Cta c;

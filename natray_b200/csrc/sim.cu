@@ -706,7 +706,7 @@ static ntr_status get_graph(Sim& S, StepGraph*& out) {
         out = &it->second;
         return NTR_OK;
     }
-    // Bound the cache: a new shape replaces the oldest when there are many.
+    // Bound the cache: a new shape replaces that of the lowest key when there are many.
     if (S.graphs.size() >= 16) {
         auto victim = S.graphs.begin();
         cudaGraphExecDestroy(victim->second.exec);
